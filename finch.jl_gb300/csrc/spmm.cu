@@ -22,20 +22,41 @@
 
 namespace fgb {
 
+// NB entries of a row, all of them stored: gathers first, then the updates in
+// storage order.  my_j/my_a: entry pb + lane of the group's current G entries.
+template <class T, int G, int V, int NB, int FM>
+__device__ __forceinline__ void pull_batch(VecT<T, V>& acc, int t, int my_j, T my_a, const T* __restrict__ Bc,
+                                           int64_t ldb, bool active, unsigned gmask, uint64_t pol) {
+  VecT<T, V> b[NB];
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    const int j = __shfl_sync(gmask, my_j, t + u, G);
+    if (active) b[u] = gather<T, V>(Bc + (int64_t)j * ldb, pol);
+  }
+#pragma unroll
+  for (int u = 0; u < NB; ++u) acc_step<T, V>(acc, __shfl_sync(gmask, my_a, t + u, G), b[u], FM);
+}
+
 // One launch = one column slab [c0, c0 + G*V) (clipped to nk) of every row.
-template <class T, class VT, class PtrT, int G, int V>
-__global__ void __launch_bounds__(256) spmm_csr_pull(
+// A row's entries are taken in batches of 8, then 4, 2 and 1, so that no
+// gather or update slot is spent on entries the row does not have: FP64 is
+// bound by its pipe (one 32-lane FMA takes 16 clocks of an SM), where a
+// predicated-off update costs as much as a real one.  200,003 rows of 10, k =
+// 33, F64: 996 us with predicated batches of 8, the contraction chosen at run
+// time and 32 lanes for the 33rd column; 198 us now (the pipe's own time for
+// 66 M FMAs is 105).
+template <class T, class VT, class PtrT, int G, int V, int FM>
+__global__ void __launch_bounds__(256, V == 1 ? 4 : 1) spmm_csr_pull(
     int64_t nrows, const PtrT* __restrict__ ptr, const int* __restrict__ idx,
     const VT* __restrict__ val, const T* __restrict__ B, int64_t ldb, T* __restrict__ C,
-    int64_t ldc, int64_t c0, int64_t nk, int base, int accumulate, int fm) {
-  constexpr int BATCH = 8;
+    int64_t ldc, int64_t c0, int64_t nk, int base, int accumulate) {
   const int lane = threadIdx.x & (G - 1);
-  const unsigned gmask =
-      G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
+  const unsigned gmask = group_mask<G>();
   const int64_t group = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int64_t ngroups = ((int64_t)gridDim.x * blockDim.x) / G;
   const int64_t col = c0 + (int64_t)lane * V;
   const bool active_col = col < nk;  // V divides nk - c0 in the vector path
+  const T* Bc = B + col;
   const uint64_t pol_stream = policy_evict_first();
   const uint64_t pol_keep = policy_evict_last();
   for (int64_t row = group; row < nrows; row += ngroups) {
@@ -56,23 +77,19 @@ __global__ void __launch_bounds__(256) spmm_csr_pull(
         my_a = load_val<T, VT>(val, pe, pol_stream);
       }
       const int cnt = (p1 - pb) < (int64_t)G ? (int)(p1 - pb) : G;
-#pragma unroll
-      for (int t0 = 0; t0 < G; t0 += BATCH) {
-        if (t0 >= cnt) break;
-        VecT<T, V> b[BATCH];
-        T a[BATCH];
-#pragma unroll
-        for (int t = 0; t < BATCH; ++t) {
-          const int src = t0 + t < G ? t0 + t : 0;
-          const int j = __shfl_sync(gmask, my_j, src, G);
-          a[t] = __shfl_sync(gmask, my_a, src, G);
-          if (t0 + t < cnt && active_col)
-            b[t] = gather<T, V>(B + (int64_t)j * ldb + col, pol_keep);
-        }
-#pragma unroll
-        for (int t = 0; t < BATCH; ++t)
-          if (t0 + t < cnt && active_col) acc_step<T, V>(acc, a[t], b[t], fm);
+      int t = 0;
+      if constexpr (G >= 8)
+        for (; t + 8 <= cnt; t += 8)
+          pull_batch<T, G, V, 8, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
+      if (t + 4 <= cnt) {
+        pull_batch<T, G, V, 4, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
+        t += 4;
       }
+      if (t + 2 <= cnt) {
+        pull_batch<T, G, V, 2, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
+        t += 2;
+      }
+      if (t < cnt) pull_batch<T, G, V, 1, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
     }
     if (active_col) store_out<T, V>(C + row * ldc + col, acc, pol_stream);
   }
@@ -109,20 +126,47 @@ __global__ void zero_rows(T* C, int64_t m, int64_t nk, int64_t ldc) {
 }
 
 template <class T, class VT, class PtrT, int G, int V>
-static int launch_pull(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk,
+static int launch_pull(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t c0, int64_t c1,
                        void* C, int64_t ldc, int accumulate, int fm, cudaStream_t s) {
   const int64_t m = A->nrows;
   const int64_t slab = (int64_t)G * V;
   const int threads = 256;
   const int grid = grid_for(m * G, threads, ctx->num_sms, 8);
-  for (int64_t c0 = 0; c0 < nk; c0 += slab) {
-    spmm_csr_pull<T, VT, PtrT, G, V><<<grid, threads, 0, s>>>(
-        m, (const PtrT*)A->ptr, (const int*)A->idx, (const VT*)A->val, (const T*)B, ldb, (T*)C,
-        ldc, c0, nk, A->index_base, accumulate, fm);
+  for (; c0 < c1; c0 += slab) {
+    if (fm == FM_NOFMA)
+      spmm_csr_pull<T, VT, PtrT, G, V, FM_NOFMA><<<grid, threads, 0, s>>>(
+          m, (const PtrT*)A->ptr, (const int*)A->idx, (const VT*)A->val, (const T*)B, ldb, (T*)C, ldc, c0, c1,
+          A->index_base, accumulate);
+    else
+      spmm_csr_pull<T, VT, PtrT, G, V, FM_FMA><<<grid, threads, 0, s>>>(
+          m, (const PtrT*)A->ptr, (const int*)A->idx, (const VT*)A->val, (const T*)B, ldb, (T*)C, ldc, c0, c1,
+          A->index_base, accumulate);
     int rc = check_launch("spmm_csr_pull");
     if (rc) return rc;
   }
   return FGB_OK;
+}
+
+// Columns [c0, nk) in slabs of `lanes` vectors; what is left over by whole
+// slabs takes the narrowest group that covers it (a 33rd column costs a
+// 4-lane launch, not another 32-lane one).
+template <class T, class VT, class PtrT, int V>
+static int pull_slabs(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk, void* C,
+                      int64_t ldc, int accumulate, int fm, int lanes, cudaStream_t s) {
+  const int G = lanes == 4 || lanes == 8 || lanes == 16 ? lanes : 32;
+  const int64_t whole = nk / (G * V) * (G * V);
+  const int64_t rest = (nk - whole + V - 1) / V;
+  auto run = [&](int g, int64_t c0, int64_t c1) {
+    switch (g) {
+      case 4: return launch_pull<T, VT, PtrT, 4, V>(ctx, A, B, ldb, c0, c1, C, ldc, accumulate, fm, s);
+      case 8: return launch_pull<T, VT, PtrT, 8, V>(ctx, A, B, ldb, c0, c1, C, ldc, accumulate, fm, s);
+      case 16: return launch_pull<T, VT, PtrT, 16, V>(ctx, A, B, ldb, c0, c1, C, ldc, accumulate, fm, s);
+      default: return launch_pull<T, VT, PtrT, 32, V>(ctx, A, B, ldb, c0, c1, C, ldc, accumulate, fm, s);
+    }
+  };
+  int rc = whole > 0 ? run(G, 0, whole) : FGB_OK;
+  if (rc == FGB_OK && rest > 0) rc = run(rest <= 4 ? 4 : rest <= 8 ? 8 : rest <= 16 ? 16 : 32, whole, nk);
+  return rc;
 }
 
 // Slab width in lanes: the whole of nk when it fits one warp, else the
@@ -133,20 +177,8 @@ static int dispatch_pull(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64
   constexpr int VN = sizeof(T) == 4 ? 4 : 2;
   const bool vec_ok = (nk % VN == 0) && (ldb % VN == 0) && (ldc % VN == 0) &&
                       ((uintptr_t)B % (VN * sizeof(T)) == 0) && ((uintptr_t)C % (VN * sizeof(T)) == 0);
-  if (vec_ok) {
-    switch (lanes) {
-      case 4: return launch_pull<T, VT, PtrT, 4, VN>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-      case 8: return launch_pull<T, VT, PtrT, 8, VN>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-      case 16: return launch_pull<T, VT, PtrT, 16, VN>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-      default: return launch_pull<T, VT, PtrT, 32, VN>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-    }
-  }
-  switch (lanes) {
-    case 4: return launch_pull<T, VT, PtrT, 4, 1>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-    case 8: return launch_pull<T, VT, PtrT, 8, 1>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-    case 16: return launch_pull<T, VT, PtrT, 16, 1>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-    default: return launch_pull<T, VT, PtrT, 32, 1>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, s);
-  }
+  if (vec_ok) return pull_slabs<T, VT, PtrT, VN>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, lanes, s);
+  return pull_slabs<T, VT, PtrT, 1>(ctx, A, B, ldb, nk, C, ldc, accumulate, fm, lanes, s);
 }
 
 static int default_lanes(int64_t nk, int vn, int64_t b_bytes) {
