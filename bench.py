@@ -1025,11 +1025,11 @@ def suite_cg_probe() -> list[dict]:
 
 def suite_spmv_adaptive() -> list[dict]:
     """The per-call CSR SpMV (no plan), FP64, on the 1M x 1M Zipf matrix
-    (16M entries) and on 4M rows of Poisson(8) entries: at these row counts
-    the library's default is the adaptive pull (one lane per row of at most
-    32 entries, a warp per longer row).  Device time per call from CUDA-graph
-    replays, and the plan autotuner's choice over 1, 4, 8 or 32 lanes per
-    row and the adaptive pull (lanes 2) with its time."""
+    (16M entries) and on 4M rows of Poisson(8) entries: the library's default
+    there samples the row lengths (lanes per row where none is long, equal
+    shares of rows and entries per warp where one is).  Device time per call
+    from CUDA-graph replays, and the plan autotuner's choice over 1, 4, 8 or
+    32 lanes per row and that pull (lanes 2) with its time."""
     import torch
 
     from finchgb import _lib as L

@@ -192,7 +192,7 @@ std::vector<Choice> candidates(const fgb_plan* p) {
     if (d.flags & FGB_FINCH_ORDER) return {Choice{1, 0}};
     for (int g : {1, 4, 8, 32}) out.push_back(Choice{g, 0});
     if (d.semiring != FGB_OR_AND && p->A.orient == FGB_CSR)
-      out.push_back(Choice{2, 0});  // the adaptive pull: one lane per short row, a warp per long one
+      out.push_back(Choice{2, 0});  // spmv_csr_auto: the pull that samples row lengths
     if (d.semiring == FGB_OR_AND && p->A.orient == FGB_CSC)
       out.push_back(Choice{0, 0});  // the warp-cooperative push over the true columns
   } else if (d.op == FGB_PLAN_SPMM) {

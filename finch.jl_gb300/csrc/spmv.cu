@@ -19,17 +19,20 @@
 // false and the pull stops a lane's scan at its first true product.  The
 // result is the full nest's, bit for bit; a sparse frontier touches only its
 // own columns' entries.
+#include <algorithm>
+#include <type_traits>
+
 #include "fgb_internal.cuh"
 #include "semiring.cuh"
 
 namespace fgb {
 
-template <int SR, class VT, class A, class PtrT, int G, bool PATTERN>
+template <int SR, class VT, class A, class PtrT, int G, bool PATTERN, int FM>
 __global__ void __launch_bounds__(256) spmv_csr_pull(int64_t nrows, const PtrT* __restrict__ ptr,
                                                      const int* __restrict__ idx,
                                                      const VT* __restrict__ val,
                                                      const A* __restrict__ x, A* __restrict__ y,
-                                                     int base, int accumulate, int fm) {
+                                                     int base, int accumulate) {
   using S = Semi<SR, A>;
   const int lane = threadIdx.x & (G - 1);
   const int64_t group = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
@@ -42,7 +45,7 @@ __global__ void __launch_bounds__(256) spmv_csr_pull(int64_t nrows, const PtrT* 
     for (int64_t p = p0 + lane; p < p1; p += G) {
       const int j = __ldg(idx + p) - base;
       const A a = PATTERN ? S::one() : to_acc<A>(val[p]);
-      acc = S::step(acc, a, __ldg(x + j), fm);
+      acc = S::step(acc, a, __ldg(x + j), FM);
       if (SR == SR_OA && acc) break;  // Bool: true absorbs every later product
     }
     if (G > 1) {
@@ -55,61 +58,246 @@ __global__ void __launch_bounds__(256) spmv_csr_pull(int64_t nrows, const PtrT* 
   }
 }
 
-// CSR pull with lanes per row chosen row by row: a warp owns 32 consecutive
-// rows; a row of at most SPMV_LONG entries is folded by its own lane (j
-// ascending, one running value, as G = 1), and the warp's longer rows are
-// then folded one after another by all 32 lanes (lane-strided, xor-shuffle
-// combine, as G = 32).  Uniform short rows run at one lane per row, the long
-// rows of a skewed matrix still spread over a warp, and the host needs no
-// row-length statistics.  Not for OR-AND (its pull stops at the first true
-// product).
+// CSR pull that suits its schedule to the row lengths it finds, with no
+// statistics from the host.  Every block reads the same 32 windows of 32
+// consecutive rows, spread over the matrix (two coalesced loads a warp each).
+//
+// No sampled row longer than `cut`: `lanes` lanes per row, grid-strided, as
+// spmv_csr_pull.  The groups of a warp are never made to meet (a ballot per
+// row would have them wait for the longest of their rows: 171 against 140 us
+// on the 4M-node graph), so a row of more than 32 * lanes entries that the
+// sample missed goes to a list.
+//
+// A longer row among them: the walk over rows and stored entries (row r sits
+// at step r + ptr[r]) is cut into equal shares, one a warp, and a warp owns
+// the rows that begin in its share: no row is split, no partial sums leave a
+// warp, and a warp that meets long rows has fewer others.  It searches ptr
+// for its first row and takes the rows 32 at a time: one of at most SPMV_LONG
+// entries by its own lane, or, where the 32 rows average SPMV_MEAN4 entries,
+// by 4 lanes (a lane's loads are uncoalesced: long enough rows pay for the
+// two shuffles); a longer row by the whole warp, one of more than SPMV_BLOCK
+// entries by way of the list.
+//
+// When a block's warps are done they share its list, the longest rows by the
+// whole block; a full list is no loss but in speed.  `ordered`
+// (FGB_FINCH_ORDER) folds every row as one running value, j ascending: a long
+// row's entries are loaded 32 at a time and folded in order by every lane.
+//
+// Bound: the gathers of x (one L1 tag a clock per SM), FP64 folds also by the
+// FP64 pipe.  GB300, per call, against rows of at most 32 entries on a lane
+// and longer ones by their warp in turn, with the contraction chosen at run
+// time: Zipf 1M x 16 FP64 286 -> 145 us with three operands in rotation, 85 in
+// a replay; uniform 4M x 8: FP64 360 -> 183, FP32 156 -> 142, Int32 min-plus
+// 149 -> 140.  Staging tiles of entries in shared memory (coalesced, every
+// row folded from there) measured 298 (FP64) and 184 (FP32) on the uniform
+// rows, and equal shares alone 194 and 162.
 constexpr int SPMV_LONG = 32;
+constexpr int SPMV_BLOCK = 2048;  // a warp alone takes 8 us for one
+constexpr int SPMV_LIST = 64;  // rows a block can leave to the end
+constexpr int SPMV_MEAN4 = 14;
 
-template <int SR, class VT, class A, class PtrT, bool PATTERN>
-__global__ void __launch_bounds__(256) spmv_csr_adaptive(int64_t nrows, const PtrT* __restrict__ ptr,
-                                                         const int* __restrict__ idx,
-                                                         const VT* __restrict__ val,
-                                                         const A* __restrict__ x, A* __restrict__ y,
-                                                         int base, int accumulate, int fm) {
+// First row whose step ptr[r] - f0 + r is at least `target` (nrows if none),
+// by the warp: 32 probes a round.
+template <class PtrT>
+__device__ __forceinline__ int64_t spmv_step_row(int64_t nrows, const PtrT* __restrict__ ptr, int64_t f0,
+                                                 int64_t entries, int64_t target, int lane) {
+  int64_t lo = target > entries ? target - entries : 0;
+  int64_t hi = target < nrows ? target : nrows;
+  if (lo > hi) lo = hi;
+  while (lo < hi) {  // warp-uniform; the span shrinks to at most span / 32 a round
+    const int64_t step = (hi - lo + 31) / 32;
+    const int64_t q = lo + lane * step;
+    const bool before = q < hi && ld_ptr(ptr, q) - f0 + q < target;
+    const int n = __popc(__ballot_sync(0xffffffffu, before));
+    if (n == 0) {
+      hi = lo;
+    } else {
+      const int64_t next = lo + n * step;
+      lo += (n - 1) * step + 1;
+      if (next < hi) hi = next;
+    }
+  }
+  return lo;
+}
+
+template <int SR, class VT, class A, class PtrT, int FM>
+__global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int64_t nrows, const PtrT* __restrict__ ptr,
+                                                        const int* __restrict__ idx,
+                                                        const VT* __restrict__ val,
+                                                        const A* __restrict__ x, A* __restrict__ y,
+                                                        int base, int accumulate, int ordered, int lanes,
+                                                        int64_t cut) {
   using S = Semi<SR, A>;
   constexpr unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r0 = warp * 32; r0 < nrows; r0 += nwarps * 32) {  // warp-uniform
-    const int64_t row = r0 + lane;
-    int64_t p0 = 0, p1 = 0;
-    if (row < nrows) {
-      p0 = ld_ptr(ptr, row) - base;
-      p1 = ld_ptr(ptr, row + 1) - base;
-    }
-    const bool is_long = p1 - p0 > SPMV_LONG;
-    if (row < nrows && !is_long) {
-      A acc = accumulate ? y[row] : S::identity();
+  constexpr int WARPS = 8;
+  __shared__ A s_red[WARPS];
+  __shared__ int64_t s_row[SPMV_LIST];  // rows left until the others are done
+  __shared__ int s_n;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t warp = (int64_t)blockIdx.x * WARPS + w;
+  const int64_t nwarps = (int64_t)gridDim.x * WARPS;
+  bool over = false;
+#pragma unroll
+  for (int u = 0; u < 32 / WARPS; ++u) {
+    const int64_t r = (int64_t)(w * (32 / WARPS) + u) * nrows / 32 + lane;
+    if (r < nrows) over |= ld_ptr(ptr, r + 1) - ld_ptr(ptr, r) > cut;
+  }
+  if (threadIdx.x == 0) s_n = 0;
+  const bool skewed = __syncthreads_or(over);
+
+  auto fold_long = [&](int64_t row, int64_t q0, int64_t q1) {  // one row by the warp
+    A acc;
+    if (ordered) {
+      acc = accumulate ? y[row] : S::identity();
+      for (int64_t q = q0; q < q1; q += 32) {
+        A a = A(0), xv = A(0);
+        if (q + lane < q1) {
+          a = to_acc<A>(val[q + lane]);
+          xv = __ldg(x + (__ldg(idx + q + lane) - base));
+        }
+        const int n = q1 - q < 32 ? (int)(q1 - q) : 32;
 #pragma unroll 4
-      for (int64_t p = p0; p < p1; ++p) {
-        const int j = __ldg(idx + p) - base;
-        const A a = PATTERN ? S::one() : to_acc<A>(val[p]);
-        acc = S::step(acc, a, __ldg(x + j), fm);
+        for (int u = 0; u < n; ++u)
+          acc = S::step(acc, __shfl_sync(FULL, a, u), __shfl_sync(FULL, xv, u), FM);
       }
-      y[row] = acc;
-    }
-    unsigned longs = __ballot_sync(FULL, is_long);
-    while (longs) {
-      const int l = __ffs(longs) - 1;
-      longs &= longs - 1;
-      const int64_t q0 = __shfl_sync(FULL, p0, l), q1 = __shfl_sync(FULL, p1, l);
-      A acc = S::identity();
+    } else {
+      acc = S::identity();
 #pragma unroll 4
-      for (int64_t p = q0 + lane; p < q1; p += 32) {
-        const int j = __ldg(idx + p) - base;
-        const A a = PATTERN ? S::one() : to_acc<A>(val[p]);
-        acc = S::step(acc, a, __ldg(x + j), fm);
+      for (int64_t q = q0 + lane; q < q1; q += 32) {
+        const int j = __ldg(idx + q) - base;
+        acc = S::step(acc, to_acc<A>(val[q]), __ldg(x + j), FM);
       }
 #pragma unroll
       for (int m = 16; m >= 1; m >>= 1) acc = S::add(acc, shfl_xor(FULL, acc, m, 32));
-      if (lane == 0) y[r0 + l] = accumulate ? S::add(y[r0 + l], acc) : acc;
+      if (accumulate) acc = S::add(y[row], acc);
     }
+    if (lane == 0) y[row] = acc;
+  };
+
+  // Leaves a row to the end; false if the list is full.
+  auto leave = [&](int64_t row) -> bool {
+    const int at = atomicAdd(&s_n, 1);
+    if (at < SPMV_LIST) s_row[at] = row;
+    return at < SPMV_LIST;
+  };
+
+  auto by_lanes = [&](auto lanes_c) {
+    constexpr int G = decltype(lanes_c)::value;
+    const int sub = lane % G;
+    const int64_t ngroups = nwarps * 32 / G;
+    for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G; row < nrows; row += ngroups) {
+      const int64_t p0 = ld_ptr(ptr, row) - base, p1 = ld_ptr(ptr, row + 1) - base;
+      if (p1 - p0 > 32 * G) {  // not sampled: the warps of the block fold it afterwards
+        int kept = 0;
+        if (sub == 0) kept = leave(row) ? 1 : 0;
+        if (__shfl_sync(group_mask<G>(), kept, 0, G)) continue;
+      }
+      A acc = G == 1 && accumulate ? y[row] : S::identity();
+#pragma unroll 4
+      for (int64_t p = p0 + sub; p < p1; p += G) {
+        const int j = __ldg(idx + p) - base;
+        acc = S::step(acc, to_acc<A>(val[p]), __ldg(x + j), FM);
+      }
+      if (G > 1) {
+#pragma unroll
+        for (int m = G / 2; m >= 1; m >>= 1) acc = S::add(acc, shfl_xor(group_mask<G>(), acc, m, G));
+        if (sub == 0) y[row] = accumulate ? S::add(y[row], acc) : acc;
+      } else {
+        y[row] = acc;
+      }
+    }
+  };
+  if (!skewed) {
+    if (lanes == 1) by_lanes(std::integral_constant<int, 1>{});
+    else if (lanes == 4) by_lanes(std::integral_constant<int, 4>{});
+    else by_lanes(std::integral_constant<int, 8>{});
+  } else {
+    const int64_t f0 = ld_ptr(ptr, 0);
+    const int64_t entries = ld_ptr(ptr, nrows) - f0;
+    const int64_t per = (entries + nrows + nwarps - 1) / nwarps;
+    const int64_t end = (warp + 1) * per;
+    int64_t r0 = spmv_step_row(nrows, ptr, f0, entries, warp * per, lane);
+    while (true) {  // warp-uniform
+      const int64_t row = r0 + lane;
+      int64_t p0 = 0, n = -1;  // -1: not this warp's row
+      if (row < nrows) {
+        p0 = ld_ptr(ptr, row) - base;
+        n = ld_ptr(ptr, row + 1) - base - p0;
+        if (p0 + base - f0 + row >= end) n = -1;
+      }
+      const bool is_long = n > SPMV_LONG;
+      const int sn = is_long ? -1 : (int)n;  // a short row's entries
+      if (!ordered && __reduce_add_sync(FULL, sn < 0 ? 0 : sn) >= 32 * SPMV_MEAN4) {
+        const int sub = lane & 3;
+#pragma unroll 1
+        for (int b = lane >> 2; b < 32; b += 8) {
+          const int64_t q0 = __shfl_sync(FULL, p0, b);
+          const int bn = __shfl_sync(FULL, sn, b);
+          A acc = S::identity();
+#pragma unroll 4
+          for (int k = sub; k < bn; k += 4) {
+            const int j = __ldg(idx + q0 + k) - base;
+            acc = S::step(acc, to_acc<A>(val[q0 + k]), __ldg(x + j), FM);
+          }
+          acc = S::add(acc, shfl_xor(FULL, acc, 2, 32));
+          acc = S::add(acc, shfl_xor(FULL, acc, 1, 32));
+          if (sub == 0 && bn >= 0) y[r0 + b] = accumulate ? S::add(y[r0 + b], acc) : acc;
+        }
+      } else if (sn >= 0) {
+        A acc = accumulate ? y[row] : S::identity();
+        const int* ix = idx + p0;
+        const VT* vx = val + p0;
+#pragma unroll 4
+        for (int k = 0; k < sn; ++k) {
+          const int j = __ldg(ix + k) - base;
+          acc = S::step(acc, to_acc<A>(vx[k]), __ldg(x + j), FM);
+        }
+        y[row] = acc;
+      }
+      unsigned longs = __ballot_sync(FULL, is_long);
+      while (longs) {
+        const int l = __ffs(longs) - 1;
+        longs &= longs - 1;
+        const int64_t q0 = __shfl_sync(FULL, p0, l), m = __shfl_sync(FULL, n, l);
+        if (m > SPMV_BLOCK && !ordered) {
+          int kept = 0;
+          if (lane == 0) kept = leave(r0 + l) ? 1 : 0;
+          if (__shfl_sync(FULL, kept, 0)) continue;
+        }
+        fold_long(r0 + l, q0, q0 + m);
+      }
+      if (__shfl_sync(FULL, (int)(n < 0), 31)) break;  // the warp's rows end here
+      r0 += 32;
+    }
+  }
+
+  __syncthreads();
+  const int left = s_n < SPMV_LIST ? s_n : SPMV_LIST;
+  for (int l = w; l < left; l += WARPS) {
+    const int64_t row = s_row[l];
+    const int64_t q0 = ld_ptr(ptr, row) - base, q1 = ld_ptr(ptr, row + 1) - base;
+    if (ordered || q1 - q0 <= SPMV_BLOCK) fold_long(row, q0, q1);
+  }
+  if (ordered) return;
+  for (int l = 0; l < left; ++l) {  // block-uniform: the longest by the whole block
+    const int64_t row = s_row[l];
+    const int64_t q0 = ld_ptr(ptr, row) - base, q1 = ld_ptr(ptr, row + 1) - base;
+    if (q1 - q0 <= SPMV_BLOCK) continue;
+    A acc = S::identity();
+#pragma unroll 4
+    for (int64_t q = q0 + threadIdx.x; q < q1; q += 32 * WARPS) {
+      const int j = __ldg(idx + q) - base;
+      acc = S::step(acc, to_acc<A>(val[q]), __ldg(x + j), FM);
+    }
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) acc = S::add(acc, shfl_xor(FULL, acc, m, 32));
+    if (lane == 0) s_red[w] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int v = 1; v < WARPS; ++v) acc = S::add(acc, s_red[v]);
+      y[row] = accumulate ? S::add(y[row], acc) : acc;
+    }
+    __syncthreads();
   }
 }
 
@@ -207,10 +395,14 @@ __global__ void fill_identity(A* __restrict__ y, int64_t n) {
 }
 
 // Lanes per fiber chosen by the plan autotuner for the calls it times and
-// captures (0 = the heuristic below, 2 = the adaptive pull); set only around
+// captures (0 = the heuristic below, 2 = spmv_csr_auto); set only around
 // those calls.
 static thread_local int t_group_override = 0;
-constexpr int SPMV_ADAPTIVE = 2;
+constexpr int SPMV_AUTO = 2;
+// Rows + entries from which a call without a plan takes spmv_csr_auto: below,
+// its sample and its list cost about what a skewed matrix gains (10,000 rows
+// of 2, FP32: 6.2 us uniform and 8.3 Zipf, against 4.2 and 16.5 by lanes).
+constexpr int64_t SPMV_AUTO_STEPS = 1 << 16;
 
 static int pick_group(double avg) {
   if (avg <= 2.0) return 1;
@@ -234,27 +426,56 @@ static int launch_typed(fgb_ctx* ctx, const fgb_sparse* A_, const void* x, void*
     int fm = FM_DEFAULT;
     if (flags & FGB_NO_FMA) fm = FM_NOFMA;
     if (flags & FGB_FMA) fm = FM_FMA;
-    int G = (flags & FGB_FINCH_ORDER) ? 1 : (t_group_override > 0 ? t_group_override : pick_group(avg));
-    // Without a plan, a matrix with rows enough to fill the device at one
-    // lane per row takes the adaptive pull: on millions of uniform rows of
-    // 2 to 24 entries one lane per row beat 4 or 8 lanes by 30-50 %
-    // (GB300, FP64), and its long rows still get a warp each.
-    if (!(flags & FGB_FINCH_ORDER) && t_group_override <= 0 && SR != SR_OA &&
-        nf >= (int64_t)ctx->num_sms * 2048)
-      G = SPMV_ADAPTIVE;
     if (nf == 0) return FGB_OK;
+    const bool ordered = flags & FGB_FINCH_ORDER;
+    int G = t_group_override > 0 ? t_group_override : ordered ? 1 : pick_group(avg);
     if constexpr (SR != SR_OA) {
-      if (G == SPMV_ADAPTIVE) {
-        const int grid = grid_for((nf + 31) / 32 * 32, threads, ctx->num_sms, 8);
-        spmv_csr_adaptive<SR, VT, A, PtrT, PATTERN><<<grid, threads, 0, s>>>(nf, ptr, idx, val, (const A*)x,
-                                                                             (A*)y, base, accumulate, fm);
-        return check_launch("spmv_csr_adaptive");
+      const int64_t steps = nf + A_->nnz;
+      if (t_group_override > 0 ? G == SPMV_AUTO : steps >= SPMV_AUTO_STEPS) {
+        // Lanes per row where no long row is sampled.  With rows enough to
+        // fill the device, one, and 4 from 14 entries a row (8-byte values:
+        // 1M x 8 rows 52 against 64 us, x 24 rows 176 against 131) or from 6
+        // (4-byte: 4M x 2 rows 41 against 74, x 8 rows 148 against 142); with
+        // fewer rows more lanes, so that more of the device works.
+        const bool many = nf >= (int64_t)ctx->num_sms * 2048;
+        const int lanes = ordered ? 1 : many ? (avg < (sizeof(A) == 8 ? SPMV_MEAN4 : 6) ? 1 : 4)
+                                             : avg <= 2.0 ? 1 : avg <= 8.0 || sizeof(A) == 8 ? 4 : 8;
+        const int64_t cut = std::max<int64_t>(SPMV_LONG, (int64_t)(4.0 * avg));
+        auto go = [&](auto fmc) {
+          auto kern = spmv_csr_auto<SR, VT, A, PtrT, decltype(fmc)::value>;
+          static const int occ = [&] {  // once per process (one device model); thread-safe
+            int o = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, threads, 0);
+            return o > 0 ? o : 1;
+          }();
+          const int64_t need = (steps + 8 * 64 - 1) / (8 * 64);  // at least 64 steps a warp
+          const int grid = (int)std::min<int64_t>(need, (int64_t)occ * ctx->num_sms);
+          kern<<<grid, threads, 0, s>>>(nf, ptr, idx, val, (const A*)x, (A*)y, base, accumulate, ordered ? 1 : 0,
+                                        lanes, cut);
+        };
+        bool unfused = false;
+        if constexpr (SR == SR_PT && std::is_floating_point<A>::value) {
+          unfused = fm == FM_NOFMA;
+          if (unfused) go(std::integral_constant<int, FM_NOFMA>{});
+        }
+        if (!unfused) go(std::integral_constant<int, FM_FMA>{});
+        return check_launch("spmv_csr_auto");
       }
     }
     int grid = grid_for(nf * G, threads, ctx->num_sms, 8);
-#define FGB_PULL(GG)                                                                    \
-  spmv_csr_pull<SR, VT, A, PtrT, GG, PATTERN><<<grid, threads, 0, s>>>(                 \
-      nf, ptr, idx, val, (const A*)x, (A*)y, base, accumulate, fm)
+#define FGB_PULL_FM(GG, FMC)                                              \
+  spmv_csr_pull<SR, VT, A, PtrT, GG, PATTERN, FMC><<<grid, threads, 0, s>>>( \
+      nf, ptr, idx, val, (const A*)x, (A*)y, base, accumulate)
+#define FGB_PULL(GG)                                                           \
+  do {                                                                         \
+    if constexpr (SR == SR_PT && std::is_floating_point<A>::value) {           \
+      if (fm == FM_NOFMA) {                                                    \
+        FGB_PULL_FM(GG, FM_NOFMA);                                             \
+        break;                                                                 \
+      }                                                                        \
+    }                                                                          \
+    FGB_PULL_FM(GG, FM_FMA);                                                   \
+  } while (0)
     switch (G) {
       case 1: FGB_PULL(1); break;
       case 4: FGB_PULL(4); break;
@@ -262,6 +483,7 @@ static int launch_typed(fgb_ctx* ctx, const fgb_sparse* A_, const void* x, void*
       default: FGB_PULL(32); break;
     }
 #undef FGB_PULL
+#undef FGB_PULL_FM
     return check_launch("spmv_csr_pull");
   }
   // CSC push

@@ -7,7 +7,7 @@ import oracle
 from finchgb import _lib as L
 from finchgb import device as dev
 from finchgb.workloads import SparseBuffers, _fibers_from_lengths, _ptr
-from helpers import to_dev, to_host, upload
+from helpers import abs_terms, assert_close, oracle_spmv, to_dev, to_host, upload
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +42,59 @@ def test_spmm_odd_widths_bit_exact(gpu_lib, dtype, nk):
         dev.spmm(A, Bd, Cd, flags=flags | L.ACCUMULATE)
         want = oracle.spmm_csr(71, 200, r.ptr, r.idx, r.val, B, C=C0.copy(), init=False, fma=fma)
         assert np.array_equal(to_host(Cd), want)
+
+
+def spmv_lengths(kind, rng):
+    if kind == "hidden":  # short rows; the long ones lie outside the sampled windows, 100 of them together
+        n = rng.integers(0, 4, 320_000)
+        n[5000:5100] = 40
+        n[[123_456, 200_111, 319_999]] = (9000, 2049, 2048)
+    elif kind == "skewed":
+        n = np.minimum(rng.zipf(1.5, 60_000), 3000)
+        n[rng.choice(60_000, 20_000, replace=False)] = 0
+        n[[0, 7, 59_999]] = (7000, 33, 32)
+    elif kind == "mid":  # rows that average over 14 entries, some long
+        n = rng.poisson(20, 8000)
+        n[:40] = 300
+    elif kind == "few":
+        n = np.array([31_000, 0, 9999, 33, 30_000])
+    else:
+        n = np.zeros(70_001, dtype=np.int64)
+    return n.astype(np.int64)
+
+
+@pytest.mark.parametrize("ptr64", [False, True])
+@pytest.mark.parametrize("kind", ["hidden", "skewed", "mid", "few", "empty"])
+def test_spmv_sampled_rows(gpu_lib, kind, ptr64):
+    """The pull that samples row lengths: equal to the nest bit for bit in
+    Finch's order (both contractions) and over an exact semiring, within the
+    bound otherwise, accumulating or not, whatever the sample missed."""
+    rng = np.random.default_rng(len(kind))
+    lengths, n = spmv_lengths(kind, rng), 40_000
+
+    def device_of(b):
+        A = upload(b)
+        if ptr64:
+            A = dev.DeviceSparse(A.nrows, A.ncols, A.ptr.long(), A.idx, A.val, A.orient, A.base)
+        return A
+
+    for dtype in (np.float64, np.float32):
+        b = csr_of_lengths(rng, lengths, n, dtype)
+        A, x = device_of(b), rng.standard_normal(n).astype(dtype)
+        y0 = rng.standard_normal(b.nrows).astype(dtype)
+        want, scale = oracle_spmv(L.PLUS_TIMES, b, x), abs_terms(b, x)
+        assert_close(to_host(dev.spmv(A, to_dev(x))), want, scale, dtype)
+        yd = to_dev(y0)
+        dev.spmv(A, to_dev(x), yd, flags=L.ACCUMULATE)
+        assert_close(to_host(yd), want.astype(np.float64) + y0, scale + np.abs(y0), dtype)
+        for fma, flag in ((True, 0), (False, L.NO_FMA)):
+            got = to_host(dev.spmv(A, to_dev(x), flags=L.FINCH_ORDER | flag))
+            assert np.array_equal(got, oracle_spmv(L.PLUS_TIMES, b, x, fma=fma))
+    b = csr_of_lengths(rng, lengths, n, np.int32)
+    x = rng.integers(-(1 << 30), 1 << 30, size=n, dtype=np.int32)
+    y0 = rng.integers(-(1 << 30), 1 << 30, size=b.nrows, dtype=np.int32)
+    want = oracle_spmv(L.MIN_PLUS, b, x)
+    assert np.array_equal(to_host(dev.spmv(device_of(b), to_dev(x), semiring=L.MIN_PLUS)), want)
+    yd = to_dev(y0)
+    dev.spmv(device_of(b), to_dev(x), yd, semiring=L.MIN_PLUS, flags=L.ACCUMULATE)
+    assert np.array_equal(to_host(yd), np.minimum(want, y0))
