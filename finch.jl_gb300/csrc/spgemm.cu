@@ -9,17 +9,20 @@
 // problem C^T = B^T A^T, whose CSR buffers are A's and B's CSC buffers.
 //
 // Per output row: an upper bound ub = sum of |R[k,:]| over the row's k picks
-// a tier -- 8 lanes (ub <= 64) or a warp (ub <= 256) with a hash table in
-// shared memory, or a block with a hash table in global scratch.  The symbolic pass inserts the
-// column keys and counts them (C's ptr); the numeric pass walks the row's k
-// in storage order, one k at a time (a barrier between them), with the
+// a tier -- one thread that merges the lists (at most 8 of them, ub <= 64), 8
+// lanes (ub <= 64) or a warp (ub <= 256) with a hash table in shared memory,
+// or a block with a hash table in global scratch.  The symbolic pass counts
+// the columns (C's ptr).  The numeric pass of the hash tiers walks the row's
+// k in storage order, one k at a time (a barrier between them), with the
 // lanes spread over R[k,:] -- every column occurs once per k, so each output
 // accumulates its products in k order without atomics, exactly Gustavson's
-// order: bit-identical to the serial nest for the same fused/unfused
-// choice.  Touched keys are stored even if their sum is zero (like the
-// workspace).  A warp writes each pair at its rank among the row's keys, so
-// small rows come out ordered; a segmented sort orders the large rows.
+// order, as the merge does: bit-identical to the serial nest for the same
+// fused/unfused choice.  Touched keys are stored even if their sum is zero
+// (like the workspace).  A warp writes each pair at its rank among the row's
+// keys, so small rows come out ordered; a segmented sort orders the large
+// rows.
 #include <cub/cub.cuh>
+#include <cuda/std/functional>
 
 #include "fgb_internal.cuh"
 #include "semiring.cuh"
@@ -40,17 +43,173 @@ static_assert(SG_WARP_SLOTS / 32 <= SG_SLOTS_PER_LANE && 2 * SG_SMALL_UB / 8 <= 
 
 __device__ __forceinline__ uint32_t sg_hash(int32_t c) { return (uint32_t)c * 2654435761u; }
 
-template <class PtrT>
-__global__ void sg_bound_k(int64_t m, const PtrT* __restrict__ lp, const int* __restrict__ li, int lbase,
-                           const PtrT* __restrict__ rp, int64_t* __restrict__ ub) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    int64_t s = 0;
-    for (int64_t q = ld_ptr(lp, r) - lbase; q < ld_ptr(lp, r + 1) - lbase; ++q) {
-      const int64_t k = __ldg(li + q) - lbase;
-      s += ld_ptr(rp, k + 1) - ld_ptr(rp, k);
+constexpr int SG_LANE_K = 8;     // lists a thread merges at most
+constexpr int SG_LANE_UB = 64;   // products of a row in the lane tier at most
+constexpr int SG_LANE_THREADS = 128;
+constexpr int SG_STAGE = 2048;   // outputs a block of the lane tier stages in shared memory
+
+template <class T>
+__device__ __forceinline__ T sg_acc(T w, T a, T b, int fm) {
+  return Semi<SR_PT, T>::step(w, a, b, fm);
+}
+
+// The lane tier, and every row's bound.  One thread per row.  A row with at
+// most SG_LANE_K stored entries and SG_LANE_UB products is merged by its
+// thread: the k lists R[k,:] are walked at once, each output the smallest
+// column at a list head, its products added in the order of k -- Gustavson's
+// order, and the columns come out ascending, so there is no table to clear,
+// probe, list and rank.  Other rows get their bound in ub[r] (-1 for a row
+// done here) and are counted by tier in n_left.
+//
+// The merge reads each list once, neighbouring rows of a banded matrix read
+// neighbouring lists, and a block whose rows are all its own writes C through
+// shared memory (a thread's own run of outputs would reach L2 as one partial
+// sector per value).  Should a list not be ascending, as SparseList has them,
+// the row is done again by selection, which needs no order.
+//
+// Bound: the chain of list heads (an L1 hit per step) and issue.  2048^2
+// 5-point matrix squared, F64, GB300: TODO
+template <class T, class PtrT, bool SYMB, int FM>
+__global__ void __launch_bounds__(SG_LANE_THREADS) sg_lane_k(
+    int64_t m, const PtrT* __restrict__ lp, const int* __restrict__ li, const T* __restrict__ lv, int lbase,
+    const PtrT* __restrict__ rp, const int* __restrict__ ri, const T* __restrict__ rv, int rbase,
+    int64_t* __restrict__ ub, unsigned long long* __restrict__ n_left, int32_t* __restrict__ cnt_out,
+    const int64_t* __restrict__ cptr, int out_base, int32_t* __restrict__ out_idx, T* __restrict__ out_val) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ int32_t s_idx[SYMB ? 1 : SG_STAGE];
+  __shared__ T s_val[SYMB ? 1 : SG_STAGE];
+  __shared__ int s_left[3];
+  const int tid = threadIdx.x;
+  const int64_t r0 = (int64_t)blockIdx.x * SG_LANE_THREADS, r = r0 + tid;
+  if (tid < 3) s_left[tid] = 0;
+  PtrT q0 = 0, q1 = 0;
+  if (r < m) {
+    q0 = __ldg(lp + r) - lbase;
+    q1 = __ldg(lp + r + 1) - lbase;
+  }
+  bool mine = r < m && q1 - q0 <= SG_LANE_K;
+  const int nk = mine ? (int)(q1 - q0) : 0;
+  const int kmax = __reduce_max_sync(FULL, nk);  // warp-uniform: lists beyond it are skipped by a branch
+  PtrT p[SG_LANE_K], e[SG_LANE_K];
+  T a[SG_LANE_K];
+#pragma unroll
+  for (int i = 0; i < SG_LANE_K; ++i) {
+    p[i] = e[i] = 0;
+    if (i < kmax && i < nk) {
+      const int k = __ldg(li + q0 + i) - lbase;
+      p[i] = __ldg(rp + k) - rbase;
+      e[i] = __ldg(rp + k + 1) - rbase;
+      if (!SYMB) a[i] = __ldg(lv + q0 + i);
     }
-    ub[r] = s;
+  }
+  int64_t u = 0;
+#pragma unroll
+  for (int i = 0; i < SG_LANE_K; ++i) u += e[i] - p[i];
+  mine = mine && u <= SG_LANE_UB;
+  __syncthreads();  // s_left is clear
+  if (r < m) {
+    if (!mine) {  // another tier's row: its whole bound, and its tier
+      if (q1 - q0 > SG_LANE_K) {
+        for (PtrT q = q0; q < q1; ++q) {
+          const int64_t k = __ldg(li + q) - lbase;
+          u += ld_ptr(rp, k + 1) - ld_ptr(rp, k);
+        }
+      }
+      atomicAdd(s_left + (u <= SG_SMALL_UB ? 0 : u <= SG_WARP_UB ? 1 : 2), 1);
+    }
+    ub[r] = mine ? -1 : u;
+  }
+  // where the row's outputs go: the block's staging array, or C
+  const bool whole = __syncthreads_and(mine || r >= m);
+  if (tid < 3 && s_left[tid]) atomicAdd(n_left + tid, (unsigned long long)s_left[tid]);
+  int32_t* o_idx = nullptr;
+  T* o_val = nullptr;
+  int room = 0;
+  int64_t c0 = 0;
+  int total = 0;
+  bool staged = false;
+  if (!SYMB) {
+    const int64_t rl = r0 + SG_LANE_THREADS < m ? r0 + SG_LANE_THREADS : m;
+    c0 = cptr[r0] - out_base;
+    const int64_t all = cptr[rl] - out_base - c0;
+    staged = whole && all <= SG_STAGE;
+    total = staged ? (int)all : 0;
+    if (mine) {
+      const int64_t at = cptr[r] - out_base;
+      room = (int)(cptr[r + 1] - out_base - at);
+      o_idx = staged ? s_idx + (at - c0) : out_idx + at;
+      o_val = staged ? s_val + (at - c0) : out_val + at;
+    }
+  }
+  if (mine) {
+    constexpr int32_t DONE = INT32_MAX;
+    PtrT h[SG_LANE_K];
+    int32_t c[SG_LANE_K];
+#pragma unroll
+    for (int i = 0; i < SG_LANE_K; ++i) {
+      h[i] = p[i];
+      c[i] = DONE;
+      if (i < kmax && h[i] < e[i]) c[i] = __ldg(ri + h[i]) - rbase;
+    }
+    int n = 0;
+    bool ascending = true;
+    while (true) {
+      int32_t col = DONE;
+#pragma unroll
+      for (int i = 0; i < SG_LANE_K; ++i)
+        if (i < kmax) col = min(col, c[i]);
+      if (col == DONE) break;
+      T w = T(0);
+#pragma unroll
+      for (int i = 0; i < SG_LANE_K; ++i) {
+        if (i < kmax && c[i] == col) {
+          if (!SYMB) w = sg_acc(w, a[i], __ldg(rv + h[i]), FM);
+          ++h[i];
+          c[i] = h[i] < e[i] ? __ldg(ri + h[i]) - rbase : DONE;
+          ascending &= c[i] > col;
+        }
+      }
+      if (!SYMB && n < room) {
+        o_idx[n] = col + out_base;
+        o_val[n] = w;
+      }
+      ++n;
+    }
+    if (!ascending) {  // by selection: the smallest column above the last, over all products
+      n = 0;
+      int32_t last = -1;
+      while (true) {
+        int32_t col = DONE;
+        for (int i = 0; i < nk; ++i) {
+          const int k = __ldg(li + q0 + i) - lbase;
+          for (PtrT t = __ldg(rp + k) - rbase; t < __ldg(rp + k + 1) - rbase; ++t) {
+            const int32_t x = __ldg(ri + t) - rbase;
+            if (x > last && x < col) col = x;
+          }
+        }
+        if (col == DONE) break;
+        if (!SYMB && n < room) {
+          T w = T(0);
+          for (int i = 0; i < nk; ++i) {
+            const int k = __ldg(li + q0 + i) - lbase;
+            for (PtrT t = __ldg(rp + k) - rbase; t < __ldg(rp + k + 1) - rbase; ++t)
+              if (__ldg(ri + t) - rbase == col) w = sg_acc(w, (T)__ldg(lv + q0 + i), __ldg(rv + t), FM);
+          }
+          o_idx[n] = col + out_base;
+          o_val[n] = w;
+        }
+        ++n;
+        last = col;
+      }
+    }
+    if (SYMB) cnt_out[r] = n;
+  }
+  if (!SYMB) {
+    __syncthreads();
+    for (int t = tid; t < total; t += SG_LANE_THREADS) {
+      out_idx[c0 + t] = s_idx[t];
+      out_val[c0 + t] = s_val[t];
+    }
   }
 }
 
@@ -92,11 +251,6 @@ __device__ __forceinline__ I sg_insert(int32_t* keys, I cap, int32_t c, bool* cr
     }
     s = (s + 1) & (cap - 1);
   }
-}
-
-template <class T>
-__device__ __forceinline__ T sg_acc(T w, T a, T b, int fm) {
-  return Semi<SR_PT, T>::step(w, a, b, fm);
 }
 
 // One row with `nthreads` cooperating threads (a warp or a block) over a
@@ -198,7 +352,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32) sg_warp_k(
     int64_t m, const int64_t* __restrict__ ub, int64_t lo, int64_t hi, const PtrT* __restrict__ lp,
     const int* __restrict__ li, const T* __restrict__ lv, int lbase, const PtrT* __restrict__ rp,
     const int* __restrict__ ri, const T* __restrict__ rv, int rbase, int fm,
-    int64_t* __restrict__ cnt_out, const int64_t* __restrict__ cptr, int out_base,
+    int32_t* __restrict__ cnt_out, const int64_t* __restrict__ cptr, int out_base,
     int32_t* __restrict__ out_idx, T* __restrict__ out_val) {
   constexpr int NG = SG_WARPS * 32 / G;      // groups per block
   constexpr int SLOTS = SG_WARP_SLOTS * G / 32;
@@ -241,7 +395,7 @@ __global__ void __launch_bounds__(SG_BLOCK) sg_block_k(
     int32_t* __restrict__ gkeys, T* __restrict__ gvals, const PtrT* __restrict__ lp,
     const int* __restrict__ li, const T* __restrict__ lv, int lbase, const PtrT* __restrict__ rp,
     const int* __restrict__ ri, const T* __restrict__ rv, int rbase, int fm,
-    int64_t* __restrict__ cnt_out, const int64_t* __restrict__ cptr, int out_base,
+    int32_t* __restrict__ cnt_out, const int64_t* __restrict__ cptr, int out_base,
     int32_t* __restrict__ out_idx, T* __restrict__ out_val) {
   __shared__ int s_cnt;
   __shared__ int64_t s_rows[SG_BLOCK];
@@ -277,12 +431,6 @@ __global__ void sg_segs_k(int64_t m, const int64_t* __restrict__ ub, const int64
   }
 }
 
-__global__ void sg_rebase_k(int64_t n, const int64_t* __restrict__ in, int base, int64_t* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = in[i] - base;
-}
-
 static inline size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct SgProblem {
@@ -291,42 +439,51 @@ struct SgProblem {
   int64_t m, n;         // rows of the CSR result, columns
 };
 
-// ub, block-tier hash offsets and the scratch for the hash tables.
+// Row bounds and counts, and what the rows beyond the lane tier need.
 struct SgScratch {
   char* mem = nullptr;
   int64_t* ub = nullptr;
   int64_t* gsize = nullptr;
   int64_t* goff = nullptr;
-  int64_t* cnt = nullptr;
+  int32_t* cnt = nullptr;
+  unsigned long long* n_left = nullptr;  // rows left by the lane tier, by tier
   int32_t* gkeys = nullptr;
   void* gvals = nullptr;
   void* cub_tmp = nullptr;
   size_t cub_bytes = 0;
 };
 
-template <class PtrT>
-static int sg_prepare(fgb_ctx* ctx, const SgProblem& P, size_t esz, SgScratch* S, cudaStream_t s) {
+static int sg_alloc(const SgProblem& P, SgScratch* S, cudaStream_t s) {
   const int64_t m = P.m;
-  size_t cub_bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, (int64_t*)nullptr, (int64_t*)nullptr, (int)(m + 1), s);
-  const size_t head = a256(8 * (m + 1)) * 4 + a256(cub_bytes);
+  size_t b1 = 0, b2 = 0;
+  cub::DeviceScan::ExclusiveSum(nullptr, b1, (int64_t*)nullptr, (int64_t*)nullptr, (int)(m + 1), s);
+  cub::DeviceScan::ExclusiveScan(nullptr, b2, (int32_t*)nullptr, (int64_t*)nullptr, cuda::std::plus<>{}, (int64_t)0,
+                                 (int)(m + 1), s);
+  const size_t cub_bytes = b1 > b2 ? b1 : b2;
+  const size_t v8 = a256(8 * (m + 1)), v4 = a256(4 * (m + 1));
   char* mem = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&mem, head, s);
+  cudaError_t e = cudaMallocAsync((void**)&mem, 3 * v8 + v4 + 256 + a256(cub_bytes), s);
   if (e != cudaSuccess) return set_error(FGB_ENOMEM, "fgb_spgemm: scratch: %s", cudaGetErrorString(e));
   S->mem = mem;
   S->ub = (int64_t*)mem;
-  S->gsize = (int64_t*)(mem + a256(8 * (m + 1)));
-  S->goff = (int64_t*)(mem + 2 * a256(8 * (m + 1)));
-  S->cnt = (int64_t*)(mem + 3 * a256(8 * (m + 1)));
-  S->cub_tmp = mem + 4 * a256(8 * (m + 1));
+  S->gsize = (int64_t*)(mem + v8);
+  S->goff = (int64_t*)(mem + 2 * v8);
+  S->cnt = (int32_t*)(mem + 3 * v8);
+  S->n_left = (unsigned long long*)(mem + 3 * v8 + v4);
+  S->cub_tmp = mem + 3 * v8 + v4 + 256;
   S->cub_bytes = cub_bytes;
-  const int grid = grid_for(m, 256, ctx->num_sms);
-  cudaMemsetAsync(S->ub + m, 0, 8, s);
-  sg_bound_k<PtrT><<<grid, 256, 0, s>>>(m, (const PtrT*)P.L->ptr, (const int*)P.L->idx, P.L->index_base,
-                                        (const PtrT*)P.R->ptr, S->ub);
-  sg_gsize_k<<<grid, 256, 0, s>>>(m + 1, S->ub, S->gsize);
-  size_t cb = cub_bytes;
-  e = cub::DeviceScan::ExclusiveSum(S->cub_tmp, cb, S->gsize, S->goff, (int)(m + 1), s);
+  e = cudaMemsetAsync(S->n_left, 0, 3 * sizeof(*S->n_left), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(S->ub + m, 0, 8, s);
+  if (e != cudaSuccess) return set_error(FGB_ECUDA, "fgb_spgemm: scratch: %s", cudaGetErrorString(e));
+  return FGB_OK;
+}
+
+// Hash tables of the block tier's rows (a host wait for their size).
+static int sg_tables(fgb_ctx* ctx, const SgProblem& P, size_t esz, SgScratch* S, cudaStream_t s) {
+  const int64_t m = P.m;
+  sg_gsize_k<<<grid_for(m, 256, ctx->num_sms), 256, 0, s>>>(m + 1, S->ub, S->gsize);
+  size_t cb = S->cub_bytes;
+  cudaError_t e = cub::DeviceScan::ExclusiveSum(S->cub_tmp, cb, S->gsize, S->goff, (int)(m + 1), s);
   int64_t total = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&total, S->goff + m, 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -348,24 +505,42 @@ static void sg_release(SgScratch* S, cudaStream_t s) {
 }
 
 template <class T, class PtrT, bool SYMB>
-static void sg_launch(fgb_ctx* ctx, const SgProblem& P, const SgScratch& S, int fm, const int64_t* cptr,
-                      int out_base, int32_t* out_idx, T* out_val, cudaStream_t s) {
+static void sg_launch_lane(const SgProblem& P, const SgScratch& S, int fm, const int64_t* cptr, int out_base,
+                           int32_t* out_idx, T* out_val, cudaStream_t s) {
+  const fgb_sparse *L = P.L, *R = P.R;
+  const int grid = (int)((P.m + SG_LANE_THREADS - 1) / SG_LANE_THREADS);
+  auto go = [&](auto kern) {
+    kern<<<grid, SG_LANE_THREADS, 0, s>>>(P.m, (const PtrT*)L->ptr, (const int*)L->idx, (const T*)L->val,
+                                          L->index_base, (const PtrT*)R->ptr, (const int*)R->idx,
+                                          (const T*)R->val, R->index_base, S.ub, S.n_left, S.cnt, cptr, out_base,
+                                          out_idx, out_val);
+  };
+  if (!SYMB && fm == FM_NOFMA) go(sg_lane_k<T, PtrT, SYMB, FM_NOFMA>);
+  else go(sg_lane_k<T, PtrT, SYMB, FM_FMA>);
+}
+
+// The rows that the lane tier left, by tier (left[t] of them).
+template <class T, class PtrT, bool SYMB>
+static void sg_launch(fgb_ctx* ctx, const SgProblem& P, const SgScratch& S, const unsigned long long* left, int fm,
+                      const int64_t* cptr, int out_base, int32_t* out_idx, T* out_val, cudaStream_t s) {
   const fgb_sparse *L = P.L, *R = P.R;
   // small rows: 8 lanes each (bound <= 64); medium: a warp each (<= 256)
-  const int g8 = grid_for(P.m, SG_WARPS * 32, ctx->num_sms, 16);
-  sg_warp_k<T, PtrT, SYMB, 8><<<g8, SG_WARPS * 32, 0, s>>>(
-      P.m, S.ub, -1, SG_SMALL_UB, (const PtrT*)L->ptr, (const int*)L->idx, (const T*)L->val,
-      L->index_base, (const PtrT*)R->ptr, (const int*)R->idx, (const T*)R->val, R->index_base, fm,
-      S.cnt, cptr, out_base, out_idx, out_val);
-  const int g32 = grid_for(P.m, SG_WARPS * 32, ctx->num_sms, 16);
-  sg_warp_k<T, PtrT, SYMB, 32><<<g32, SG_WARPS * 32, 0, s>>>(
-      P.m, S.ub, SG_SMALL_UB, SG_WARP_UB, (const PtrT*)L->ptr, (const int*)L->idx, (const T*)L->val,
-      L->index_base, (const PtrT*)R->ptr, (const int*)R->idx, (const T*)R->val, R->index_base, fm,
-      S.cnt, cptr, out_base, out_idx, out_val);
-  sg_block_k<T, PtrT, SYMB><<<ctx->num_sms * 4, SG_BLOCK, 0, s>>>(
-      P.m, S.ub, S.goff, S.gkeys, (T*)S.gvals, (const PtrT*)L->ptr, (const int*)L->idx,
-      (const T*)L->val, L->index_base, (const PtrT*)R->ptr, (const int*)R->idx, (const T*)R->val,
-      R->index_base, fm, S.cnt, cptr, out_base, out_idx, out_val);
+  const int g = grid_for(P.m, SG_WARPS * 32, ctx->num_sms, 16);
+  if (left[0])
+    sg_warp_k<T, PtrT, SYMB, 8><<<g, SG_WARPS * 32, 0, s>>>(
+        P.m, S.ub, -1, SG_SMALL_UB, (const PtrT*)L->ptr, (const int*)L->idx, (const T*)L->val,
+        L->index_base, (const PtrT*)R->ptr, (const int*)R->idx, (const T*)R->val, R->index_base, fm,
+        S.cnt, cptr, out_base, out_idx, out_val);
+  if (left[1])
+    sg_warp_k<T, PtrT, SYMB, 32><<<g, SG_WARPS * 32, 0, s>>>(
+        P.m, S.ub, SG_SMALL_UB, SG_WARP_UB, (const PtrT*)L->ptr, (const int*)L->idx, (const T*)L->val,
+        L->index_base, (const PtrT*)R->ptr, (const int*)R->idx, (const T*)R->val, R->index_base, fm,
+        S.cnt, cptr, out_base, out_idx, out_val);
+  if (left[2])
+    sg_block_k<T, PtrT, SYMB><<<ctx->num_sms * 4, SG_BLOCK, 0, s>>>(
+        P.m, S.ub, S.goff, S.gkeys, (T*)S.gvals, (const PtrT*)L->ptr, (const int*)L->idx,
+        (const T*)L->val, L->index_base, (const PtrT*)R->ptr, (const int*)R->idx, (const T*)R->val,
+        R->index_base, fm, S.cnt, cptr, out_base, out_idx, out_val);
 }
 
 static int sg_problem(const fgb_sparse* A, const fgb_sparse* B, SgProblem* P, const char* who) {
@@ -396,29 +571,46 @@ extern "C" int fgb_spgemm_symbolic(fgb_ctx* ctx, const fgb_sparse* A, const fgb_
   if (!rc) rc = sg_problem(A, B, &P, "fgb_spgemm_symbolic");
   if (rc) return rc;
   cudaStream_t s = pick_stream(ctx, stream);
+  const bool i32 = A->ptr_t == FGB_I32;
   SgScratch S;
-  rc = A->ptr_t == FGB_I32 ? sg_prepare<int32_t>(ctx, P, 1, &S, s) : sg_prepare<int64_t>(ctx, P, 1, &S, s);
+  rc = sg_alloc(P, &S, s);
   if (rc) {
     sg_release(&S, s);
     return rc;
   }
-  cudaMemsetAsync(S.cnt + P.m, 0, 8, s);
-  if (A->ptr_t == FGB_I32)
-    sg_launch<float, int32_t, true>(ctx, P, S, 0, nullptr, 0, nullptr, nullptr, s);
-  else
-    sg_launch<float, int64_t, true>(ctx, P, S, 0, nullptr, 0, nullptr, nullptr, s);
-  size_t cb = S.cub_bytes;
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(S.cub_tmp, cb, S.cnt, c_ptr, (int)(P.m + 1), s);
-  // C's ptr in A's index base
-  if (e == cudaSuccess && A->index_base != 0) {
-    sg_rebase_k<<<grid_for(P.m + 1, 256, ctx->num_sms), 256, 0, s>>>(P.m + 1, c_ptr, -A->index_base, c_ptr);
+  // The counts are scanned before the host knows whether the lane tier left
+  // any row: one wait where it left none, and a second scan where it did.
+  unsigned long long left[3] = {0, 0, 0};
+  int64_t total = 0;
+  cudaError_t e = cudaMemsetAsync(S.cnt, 0, 4 * (P.m + 1), s);
+  if (e == cudaSuccess && P.m > 0) {
+    if (i32) sg_launch_lane<float, int32_t, true>(P, S, 0, nullptr, 0, nullptr, nullptr, s);
+    else sg_launch_lane<float, int64_t, true>(P, S, 0, nullptr, 0, nullptr, nullptr, s);
     e = cudaGetLastError();
   }
-  int64_t total = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&total, c_ptr + P.m, 8, cudaMemcpyDeviceToHost, s);
-  sg_release(&S, s);
+  auto scan = [&]() {  // C's ptr, in A's index base
+    size_t cb = S.cub_bytes;
+    if (e == cudaSuccess)
+      e = cub::DeviceScan::ExclusiveScan(S.cub_tmp, cb, S.cnt, c_ptr, cuda::std::plus<>{}, (int64_t)A->index_base,
+                                         (int)(P.m + 1), s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&total, c_ptr + P.m, 8, cudaMemcpyDeviceToHost, s);
+  };
+  scan();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(left, S.n_left, sizeof(left), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && (left[0] || left[1] || left[2])) {
+    if (left[2]) rc = sg_tables(ctx, P, 1, &S, s);
+    if (rc) {
+      sg_release(&S, s);
+      return rc;
+    }
+    if (i32) sg_launch<float, int32_t, true>(ctx, P, S, left, 0, nullptr, 0, nullptr, nullptr, s);
+    else sg_launch<float, int64_t, true>(ctx, P, S, left, 0, nullptr, 0, nullptr, nullptr, s);
+    e = cudaGetLastError();
+    scan();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  }
+  sg_release(&S, s);
   if (e != cudaSuccess) return set_error(FGB_ECUDA, "fgb_spgemm_symbolic: %s", cudaGetErrorString(e));
   *nnz_c = total - A->index_base;
   return FGB_OK;
@@ -443,7 +635,7 @@ extern "C" int fgb_spgemm_numeric(fgb_ctx* ctx, const fgb_sparse* A, const fgb_s
   cudaStream_t s = pick_stream(ctx, stream);
   SgScratch S;
   const size_t esz = dtype == FGB_F64 ? 8 : 4;
-  rc = A->ptr_t == FGB_I32 ? sg_prepare<int32_t>(ctx, P, esz, &S, s) : sg_prepare<int64_t>(ctx, P, esz, &S, s);
+  rc = sg_alloc(P, &S, s);
   if (rc) {
     sg_release(&S, s);
     return rc;
@@ -451,19 +643,34 @@ extern "C" int fgb_spgemm_numeric(fgb_ctx* ctx, const fgb_sparse* A, const fgb_s
   const int64_t* cptr = (const int64_t*)C->ptr;
   int32_t* cidx = (int32_t*)C->idx;
   const int ob = C->index_base;
-#define SG_NUM(T, PT) sg_launch<T, PT, false>(ctx, P, S, fm, cptr, ob, cidx, (T*)C->val, s)
-  if (dtype == FGB_F64) {
-    if (A->ptr_t == FGB_I32) SG_NUM(double, int32_t); else SG_NUM(double, int64_t);
-  } else {
-    if (A->ptr_t == FGB_I32) SG_NUM(float, int32_t); else SG_NUM(float, int64_t);
+  const bool i32 = A->ptr_t == FGB_I32;
+  unsigned long long left[3] = {0, 0, 0};
+#define SG_NUM(FN, ...)                                                                              \
+  do {                                                                                               \
+    if (dtype == FGB_F64) {                                                                          \
+      if (i32) FN<double, int32_t, false>(__VA_ARGS__, fm, cptr, ob, cidx, (double*)C->val, s);      \
+      else FN<double, int64_t, false>(__VA_ARGS__, fm, cptr, ob, cidx, (double*)C->val, s);          \
+    } else {                                                                                         \
+      if (i32) FN<float, int32_t, false>(__VA_ARGS__, fm, cptr, ob, cidx, (float*)C->val, s);        \
+      else FN<float, int64_t, false>(__VA_ARGS__, fm, cptr, ob, cidx, (float*)C->val, s);            \
+    }                                                                                                \
+  } while (0)
+  if (P.m > 0) SG_NUM(sg_launch_lane, P, S);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(left, S.n_left, sizeof(left), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && (left[0] || left[1] || left[2])) {
+    if (left[2]) rc = sg_tables(ctx, P, esz, &S, s);
+    if (rc) {
+      sg_release(&S, s);
+      return rc;
+    }
+    SG_NUM(sg_launch, ctx, P, S, left);
+    e = cudaGetLastError();
   }
 #undef SG_NUM
-  cudaError_t e = cudaGetLastError();
   // order the large rows' columns (keys compared with the base added: same order)
-  int64_t n_big = 0;
-  if (e == cudaSuccess && C->nnz > 0) e = cudaMemcpyAsync(&n_big, S.goff + P.m, 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess && C->nnz > 0 && n_big > 0) {
+  if (e == cudaSuccess && C->nnz > 0 && left[2]) {
     int64_t* seg = nullptr;  // begin offsets, then end offsets (0-based)
     int32_t* k2 = nullptr;
     void* v2 = nullptr;
@@ -503,7 +710,7 @@ extern "C" int fgb_spgemm_numeric(fgb_ctx* ctx, const fgb_sparse* A, const fgb_s
     if (seg) cudaFreeAsync(seg, s);
   }
   sg_release(&S, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && (left[0] || left[1] || left[2])) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return set_error(FGB_ECUDA, "fgb_spgemm_numeric: %s", cudaGetErrorString(e));
   return FGB_OK;
 }

@@ -98,3 +98,28 @@ def test_spmv_sampled_rows(gpu_lib, kind, ptr64):
     yd = to_dev(y0)
     dev.spmv(device_of(b), to_dev(x), yd, semiring=L.MIN_PLUS, flags=L.ACCUMULATE)
     assert np.array_equal(to_host(yd), np.minimum(want, y0))
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shape", ["edges", "wide", "ragged"])
+def test_spgemm_merged_rows(gpu_lib, dtype, shape):
+    """Rows that one thread merges, beside rows of the hash tiers: 0 to 10
+    lists, bounds about 64, blocks of 128 rows with more outputs than the
+    staging array holds, a last block that is not full.  The product is the
+    serial nest's bit for bit, also where the lists are not ascending."""
+    rng = np.random.default_rng(len(shape))
+    if shape == "edges":
+        la, lb, n = np.arange(700) % 11, np.full(300, 8), 5000
+    elif shape == "wide":  # 8 lists of 8: 64 products, nearly as many outputs
+        la, lb, n = np.full(257, 8), np.full(300, 8), 100_000
+    else:
+        la, lb, n = rng.integers(0, 9, 1000), rng.integers(0, 30, 300), 900
+    A, B = csr_of_lengths(rng, la, 300, dtype), csr_of_lengths(rng, lb, n, dtype)
+    for fma, flags in ((True, 0), (False, L.NO_FMA)):
+        ptr, idx, val = dev.spgemm(upload(A), upload(B), flags=flags).to_host()
+        wp, wi, wv = oracle.spgemm_csr(la.size, n, A.ptr, A.idx, A.val, B.ptr, B.idx, B.val, fma=fma)
+        assert np.array_equal(ptr, wp) and np.array_equal(idx, wi) and np.array_equal(val, wv)
+    order = np.lexsort((rng.random(B.nnz), np.repeat(np.arange(300), lb)))  # each list shuffled
+    S = SparseBuffers(300, n, B.ptr, B.idx[order], B.val[order], "csr")
+    ptr2, idx2, val2 = dev.spgemm(upload(A), upload(S), flags=L.NO_FMA).to_host()
+    assert np.array_equal(ptr2, ptr) and np.array_equal(idx2, idx) and np.array_equal(val2, val)
