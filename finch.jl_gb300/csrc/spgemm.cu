@@ -23,6 +23,7 @@
 // rows.
 #include <cub/cub.cuh>
 #include <cuda/std/functional>
+#include <type_traits>
 
 #include "fgb_internal.cuh"
 #include "semiring.cuh"
@@ -45,8 +46,8 @@ __device__ __forceinline__ uint32_t sg_hash(int32_t c) { return (uint32_t)c * 26
 
 constexpr int SG_LANE_K = 8;     // lists a thread merges at most
 constexpr int SG_LANE_UB = 64;   // products of a row in the lane tier at most
-constexpr int SG_LANE_THREADS = 128;
-constexpr int SG_STAGE = 2048;   // outputs a block of the lane tier stages in shared memory
+constexpr int SG_LANE_THREADS = 64;
+constexpr int SG_STAGE = 14 * SG_LANE_THREADS;   // outputs a block of the lane tier stages in shared memory
 
 template <class T>
 __device__ __forceinline__ T sg_acc(T w, T a, T b, int fm) {
@@ -67,10 +68,15 @@ __device__ __forceinline__ T sg_acc(T w, T a, T b, int fm) {
 // sector per value).  Should a list not be ascending, as SparseList has them,
 // the row is done again by selection, which needs no order.
 //
-// Bound: the chain of list heads (an L1 hit per step) and issue.  2048^2
-// 5-point matrix squared, F64, GB300: TODO
+// Bound: symbolic, issue (81 % with all lists predicated, hence the build for
+// 5 lists); numeric, L1 misses on the way to the next head (38 % hits: the
+// lists of the resident warps and the staging arrays share it).  2048^2
+// 5-point matrix squared, F64, GB300, the whole product: 3675 us with hash
+// tables, 898 with 8 predicated lists in blocks of 128 rows, 782 with the
+// build for 5, 712 in blocks of 64 with 14 staged outputs a row, 695 with the
+// heads' values loaded ahead (946 with no staging).
 template <class T, class PtrT, bool SYMB, int FM>
-__global__ void __launch_bounds__(SG_LANE_THREADS) sg_lane_k(
+__global__ void __launch_bounds__(SG_LANE_THREADS, 12) sg_lane_k(
     int64_t m, const PtrT* __restrict__ lp, const int* __restrict__ li, const T* __restrict__ lv, int lbase,
     const PtrT* __restrict__ rp, const int* __restrict__ ri, const T* __restrict__ rv, int rbase,
     int64_t* __restrict__ ub, unsigned long long* __restrict__ n_left, int32_t* __restrict__ cnt_out,
@@ -89,13 +95,13 @@ __global__ void __launch_bounds__(SG_LANE_THREADS) sg_lane_k(
   }
   bool mine = r < m && q1 - q0 <= SG_LANE_K;
   const int nk = mine ? (int)(q1 - q0) : 0;
-  const int kmax = __reduce_max_sync(FULL, nk);  // warp-uniform: lists beyond it are skipped by a branch
+  const int kmax = __reduce_max_sync(FULL, nk);
   PtrT p[SG_LANE_K], e[SG_LANE_K];
   T a[SG_LANE_K];
 #pragma unroll
   for (int i = 0; i < SG_LANE_K; ++i) {
     p[i] = e[i] = 0;
-    if (i < kmax && i < nk) {
+    if (i < nk) {
       const int k = __ldg(li + q0 + i) - lbase;
       p[i] = __ldg(rp + k) - rbase;
       e[i] = __ldg(rp + k + 1) - rbase;
@@ -141,40 +147,47 @@ __global__ void __launch_bounds__(SG_LANE_THREADS) sg_lane_k(
       o_val = staged ? s_val + (at - c0) : out_val + at;
     }
   }
+  constexpr int32_t DONE = INT32_MAX;
   if (mine) {
-    constexpr int32_t DONE = INT32_MAX;
-    PtrT h[SG_LANE_K];
-    int32_t c[SG_LANE_K];
-#pragma unroll
-    for (int i = 0; i < SG_LANE_K; ++i) {
-      h[i] = p[i];
-      c[i] = DONE;
-      if (i < kmax && h[i] < e[i]) c[i] = __ldg(ri + h[i]) - rbase;
-    }
     int n = 0;
     bool ascending = true;
-    while (true) {
-      int32_t col = DONE;
-#pragma unroll
-      for (int i = 0; i < SG_LANE_K; ++i)
-        if (i < kmax) col = min(col, c[i]);
-      if (col == DONE) break;
-      T w = T(0);
-#pragma unroll
-      for (int i = 0; i < SG_LANE_K; ++i) {
-        if (i < kmax && c[i] == col) {
-          if (!SYMB) w = sg_acc(w, a[i], __ldg(rv + h[i]), FM);
-          ++h[i];
-          c[i] = h[i] < e[i] ? __ldg(ri + h[i]) - rbase : DONE;
-          ascending &= c[i] > col;
+    auto merge = [&](auto km) {  // the first KM lists
+      constexpr int KM = decltype(km)::value;
+      int32_t c[KM];
+      T v[KM];  // the heads' columns and values, loaded when a list advances
+      auto head = [&](int i) {
+        c[i] = DONE;
+        if (p[i] < e[i]) {
+          c[i] = __ldg(ri + p[i]) - rbase;
+          if (!SYMB) v[i] = __ldg(rv + p[i]);
         }
+      };
+#pragma unroll
+      for (int i = 0; i < KM; ++i) head(i);
+      while (true) {
+        int32_t col = c[0];
+#pragma unroll
+        for (int i = 1; i < KM; ++i) col = min(col, c[i]);
+        if (col == DONE) break;
+        T w = T(0);
+#pragma unroll
+        for (int i = 0; i < KM; ++i) {
+          if (c[i] == col) {
+            if (!SYMB) w = sg_acc(w, a[i], v[i], FM);
+            ++p[i];
+            head(i);
+            ascending &= c[i] > col;
+          }
+        }
+        if (!SYMB && n < room) {
+          o_idx[n] = col + out_base;
+          o_val[n] = w;
+        }
+        ++n;
       }
-      if (!SYMB && n < room) {
-        o_idx[n] = col + out_base;
-        o_val[n] = w;
-      }
-      ++n;
-    }
+    };
+    if (kmax <= 5) merge(std::integral_constant<int, 5>{});  // warp-uniform
+    else merge(std::integral_constant<int, SG_LANE_K>{});
     if (!ascending) {  // by selection: the smallest column above the last, over all products
       n = 0;
       int32_t last = -1;
