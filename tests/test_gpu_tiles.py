@@ -123,3 +123,51 @@ def test_spgemm_merged_rows(gpu_lib, dtype, shape):
     S = SparseBuffers(300, n, B.ptr, B.idx[order], B.val[order], "csr")
     ptr2, idx2, val2 = dev.spgemm(upload(A), upload(S), flags=L.NO_FMA).to_host()
     assert np.array_equal(ptr2, ptr) and np.array_equal(idx2, idx) and np.array_equal(val2, val)
+
+
+def ewise_pair(kind, rng, dtype):
+    """Two matrices of one shape that share about half their places."""
+    n = 20_000
+    if kind == "short":  # several staged tiles, the last one not full
+        la = rng.integers(0, 17, 3001)
+    elif kind == "long":  # long pairs in staged tiles and beyond them
+        la = rng.integers(0, 6, 500)
+        la[[3, 4, 100, 499]] = (33, 64, 700, 9000)
+    elif kind == "one":
+        la = np.array([5000])
+    else:  # nothing, or nothing in one of the two
+        la = np.zeros(200, dtype=np.int64)
+        la[7] = 40
+    A = csr_of_lengths(rng, la, n, dtype)
+    f = np.repeat(np.arange(la.size), la)
+    keep = rng.random(A.nnz) < 0.5
+    key = np.unique(np.concatenate([f[keep] * n + A.idx[keep] - 1,
+                                    rng.integers(0, la.size * n, int((~keep).sum()) if kind != "none" else 0)]))
+    lb = np.bincount(key // n, minlength=la.size)
+    B = csr_of_lengths(rng, lb, n, dtype)
+    B.idx = key % n + 1
+    return A, B
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32, np.int32, np.int64])
+@pytest.mark.parametrize("kind", ["short", "long", "one", "none"])
+def test_ewise_tiles(gpu_lib, kind, dtype):
+    """Merges of short pairs (a thread each, staged) and long ones (a warp
+    each, staged or not), with ptr widths and index bases of their own:
+    structure and values equal the two-finger merge's; sums are within the
+    bound, over every dimension."""
+    rng = np.random.default_rng(len(kind))
+    A, B = ewise_pair(kind, rng, dtype)
+    for a, b in ((A, B), (B, A)):
+        da, db = upload(a), upload(b)
+        db = dev.DeviceSparse(db.nrows, db.ncols, db.ptr.long() - 1, db.idx - 1, db.val, "csr", 0)
+        for op in (L.EW_MUL, L.EW_ADD):
+            ptr, idx, val = dev.ewise(op, da, db).to_host()
+            wp, wi, wv = oracle.ewise(op, a.nrows, a.ptr, a.idx, a.val, b.ptr, b.idx, b.val)
+            assert np.array_equal(ptr, wp) and np.array_equal(idx, wi) and np.array_equal(val, wv)
+        if np.dtype(dtype).kind == "f":
+            for dims in (0, 1, 2):
+                args = (dims, a.nrows, a.ncols, a.ptr, a.idx)
+                want = oracle.ewise_reduce(*args, a.val, b.ptr, b.idx, b.val)
+                scale = oracle.ewise_reduce(*args, np.abs(a.val), b.ptr, b.idx, np.abs(b.val))
+                assert_close(to_host(dev.ewise_reduce(dims, da, db)), want, scale, dtype)
