@@ -74,17 +74,28 @@ __device__ __forceinline__ bool row_is_light(const RowBands& rb, int P, int T) {
   return true;
 }
 
-// Per row: virtual rows, partial-sum slots, fix-up segments (a row's slots in
-// runs of at most VR_SEG), whether it is a long row (more than one segment:
-// its segment sums are combined by a second pass) and its segment sums; per
-// band (atomically, into band_cnt): the virtual rows of that band.
+// Per row, two counts to a 64-bit word so that two scans place everything
+// (each count's total stays below 2^32): virtual rows and partial-sum slots
+// (rows_slots), fix-up segments (a row's slots in runs of at most VR_SEG) and
+// segment sums (segs_sums; a long row's, one with more than one segment,
+// combined by a second pass).  Totals: virtual rows per band, then long rows.
+// They are summed by block first: an atomic per thread on one address took
+// 200 of the launch's 206 us on the 1M-row matrix.
+__device__ __forceinline__ int64_t vr_pack(int64_t lo, int64_t hi) { return lo | hi << 32; }
+__host__ __device__ __forceinline__ int64_t vr_lo(int64_t w) { return w & 0xffffffffll; }
+__host__ __device__ __forceinline__ int64_t vr_hi(int64_t w) { return (int64_t)((uint64_t)w >> 32); }
+
 template <class PtrT>
-__global__ void vrow_count_k(int64_t nrows, const PtrT* __restrict__ ptr, const int* __restrict__ idx,
-                             int base, int T, int P, int64_t W, int64_t* __restrict__ nv,
-                             int64_t* __restrict__ nl, int64_t* __restrict__ nseg,
-                             int64_t* __restrict__ nlong, int64_t* __restrict__ nss,
-                             unsigned long long* __restrict__ band_cnt) {
-  unsigned long long mine[VR_MAX_BANDS] = {};
+__global__ void __launch_bounds__(256) vrow_count_k(int64_t nrows, const PtrT* __restrict__ ptr,
+                                                    const int* __restrict__ idx, int base, int T, int P, int64_t W,
+                                                    int64_t* __restrict__ rows_slots,
+                                                    int64_t* __restrict__ segs_sums,
+                                                    unsigned long long* __restrict__ totals) {
+  __shared__ unsigned long long s_tot[VR_MAX_BANDS + 1];
+  if (threadIdx.x <= VR_MAX_BANDS) s_tot[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned mine[VR_MAX_BANDS] = {};
+  unsigned nlong = 0;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nrows;
        r += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b0 = ld_ptr(ptr, r) - base;
@@ -111,19 +122,23 @@ __global__ void vrow_count_k(int64_t nrows, const PtrT* __restrict__ ptr, const 
         const int64_t lb = rb.pos[b + 1] - rb.pos[b];
         const int64_t c = (lb + T - 1) / T;
         nch += c;
-        mine[b] += (unsigned long long)c;
+        mine[b] += (unsigned)c;
       }
       slots = nch - 1;
     }
     const int64_t segs = (slots + VR_SEG - 1) / VR_SEG;
-    nv[r] = nch;
-    nl[r] = slots;
-    nseg[r] = segs;
-    nlong[r] = segs > 1 ? 1 : 0;
-    nss[r] = segs > 1 ? segs : 0;
+    rows_slots[r] = vr_pack(nch, slots);
+    segs_sums[r] = vr_pack(segs, segs > 1 ? segs : 0);
+    nlong += segs > 1;
   }
-  for (int b = 0; b < P; ++b)
-    if (mine[b]) atomicAdd(band_cnt + b, mine[b]);
+  auto add = [&](int t, unsigned v) {
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(s_tot + t, (unsigned long long)v);
+  };
+  for (int b = 0; b < P; ++b) add(b, mine[b]);
+  add(VR_MAX_BANDS, nlong);
+  __syncthreads();
+  if (threadIdx.x <= VR_MAX_BANDS && s_tot[threadIdx.x]) atomicAdd(totals + threadIdx.x, s_tot[threadIdx.x]);
 }
 
 __device__ __forceinline__ uint8_t vrow_class(int64_t len) {
@@ -133,14 +148,14 @@ __device__ __forceinline__ uint8_t vrow_class(int64_t len) {
 }
 
 // The virtual rows of every row (unsorted, with their band and length-class
-// keys) and its fix-up records.  soff/goff/ssoff: exclusive scans of the
-// segments, the long rows and the segment sums (vrow_count_k).  Record w:
+// keys) and its fix-up records, from the exclusive scans of vrow_count_k's
+// words; the long rows are listed in any order (each is summed by itself).
+// Record w:
 // -1 writes C, -2 adds to C (a light row's later band), >= 0 a partial slot.
 template <class PtrT>
 __global__ void vrow_fill_k(int64_t nrows, const PtrT* __restrict__ ptr, const int* __restrict__ idx,
-                            int base, int T, int P, int64_t W, const int64_t* __restrict__ voff,
-                            const int64_t* __restrict__ loff, const int64_t* __restrict__ soff,
-                            const int64_t* __restrict__ goff, const int64_t* __restrict__ ssoff,
+                            int base, int T, int P, int64_t W, const int64_t* __restrict__ rows_slots,
+                            const int64_t* __restrict__ segs_sums, unsigned long long* __restrict__ nlong,
                             uint8_t* __restrict__ key, int32_t* __restrict__ ord,
                             int4* __restrict__ unsorted, int4* __restrict__ seg, int4* __restrict__ lrow) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nrows;
@@ -153,7 +168,7 @@ __global__ void vrow_fill_k(int64_t nrows, const PtrT* __restrict__ ptr, const i
       rb.pos[0] = 0;
       rb.pos[1] = len;
     }
-    const int64_t v0 = voff[r], l0 = loff[r];
+    const int64_t at = rows_slots[r], v0 = vr_lo(at), l0 = vr_hi(at);
     int64_t c = 0;  // virtual rows written so far
     auto emit = [&](int b, int64_t first, int64_t clen, int w) {
       const int64_t v = v0 + c;
@@ -178,17 +193,18 @@ __global__ void vrow_fill_k(int64_t nrows, const PtrT* __restrict__ ptr, const i
           emit(b, f, clen, c == 0 ? -1 : (int)(l0 + c - 1));
         }
     }
-    const int64_t slots = loff[r + 1] - l0, s0 = soff[r], segs = soff[r + 1] - s0;
+    const int64_t slots = vr_hi(rows_slots[r + 1]) - l0, sg = segs_sums[r], s0 = vr_lo(sg);
+    const int64_t segs = vr_lo(segs_sums[r + 1]) - s0;
     if (segs == 1) {
       seg[s0] = make_int4((int)r, (int)l0, (int)slots, -1);
     } else if (segs > 1) {
-      const int64_t ss0 = ssoff[r];
+      const int64_t ss0 = vr_hi(sg);
       for (int64_t g = 0; g < segs; ++g) {
         const int64_t first = g * VR_SEG;
         const int64_t n = slots - first < VR_SEG ? slots - first : VR_SEG;
         seg[s0 + g] = make_int4((int)r, (int)(l0 + first), (int)n, (int)(ss0 + g));
       }
-      lrow[goff[r]] = make_int4((int)r, (int)ss0, (int)segs, 0);
+      lrow[atomicAdd(nlong, 1ull)] = make_int4((int)r, (int)ss0, (int)segs, 0);
     }
   }
 }
@@ -481,19 +497,14 @@ static int vrow_build_t(fgb_ctx* ctx, const fgb_sparse* A, int T, int P, VrowSch
   const int grid = grid_for(nrows, 256, ctx->num_sms);
   // Temporaries come from the stream-ordered pool (kept mapped across calls);
   // the schedule itself too when `pooled` (a schedule built for one call).
-  int64_t *cnt_v = nullptr, *cnt_l = nullptr, *voff = nullptr, *loff = nullptr;
-  int64_t *cnt_s = nullptr, *cnt_g = nullptr, *cnt_ss = nullptr, *soff = nullptr, *goff = nullptr,
-          *ssoff = nullptr;
+  int64_t* words = nullptr;  // two counts and their two scans
   void* cub_tmp = nullptr;
   char* tmp = nullptr;
   char* mem = nullptr;
-  unsigned long long* band_cnt = nullptr;
   size_t cub_bytes = 0, b2 = 0;
   cudaError_t e = cudaSuccess;
   auto release = [&](bool keep_schedule) {
-    for (void* q : {(void*)cnt_v, (void*)cnt_l, (void*)voff, (void*)loff, (void*)cnt_s, (void*)cnt_g,
-                    (void*)cnt_ss, (void*)soff, (void*)goff, (void*)ssoff, cub_tmp, (void*)tmp,
-                    (void*)band_cnt})
+    for (void* q : {(void*)words, cub_tmp, (void*)tmp})
       if (q) cudaFreeAsync(q, s);
     if (!keep_schedule && mem) {
       if (pooled) cudaFreeAsync(mem, s);
@@ -506,37 +517,28 @@ static int vrow_build_t(fgb_ctx* ctx, const fgb_sparse* A, int T, int P, VrowSch
     return set_error(e == cudaErrorMemoryAllocation ? FGB_ENOMEM : FGB_ECUDA, "vrow schedule: %s: %s",
                      what, cudaGetErrorString(e));
   };
-  const size_t rows_bytes = sizeof(int64_t) * (nrows + 1);
-  if ((e = cudaMallocAsync((void**)&cnt_v, rows_bytes, s)) != cudaSuccess) return fail("alloc");
-  if ((e = cudaMallocAsync((void**)&cnt_l, rows_bytes, s)) != cudaSuccess) return fail("alloc");
-  if ((e = cudaMallocAsync((void**)&voff, rows_bytes, s)) != cudaSuccess) return fail("alloc");
-  if ((e = cudaMallocAsync((void**)&loff, rows_bytes, s)) != cudaSuccess) return fail("alloc");
-  for (int64_t** q : {&cnt_s, &cnt_g, &cnt_ss, &soff, &goff, &ssoff})
-    if ((e = cudaMallocAsync((void**)q, rows_bytes, s)) != cudaSuccess) return fail("alloc");
-  if ((e = cudaMallocAsync((void**)&band_cnt, sizeof(unsigned long long) * VR_MAX_BANDS, s)) != cudaSuccess)
-    return fail("alloc");
-  cudaMemsetAsync(band_cnt, 0, sizeof(unsigned long long) * VR_MAX_BANDS, s);
-  for (int64_t* q : {cnt_v, cnt_l, cnt_s, cnt_g, cnt_ss}) cudaMemsetAsync(q + nrows, 0, sizeof(int64_t), s);
+  constexpr int NTOT = VR_MAX_BANDS + 2;  // vrow_count_k's totals, then the fill's long-row counter
+  const int64_t nw = nrows + 1;
+  if ((e = cudaMallocAsync((void**)&words, sizeof(int64_t) * (4 * nw + NTOT), s)) != cudaSuccess) return fail("alloc");
+  int64_t *cnt_a = words, *cnt_b = words + nw, *off_a = words + 2 * nw, *off_b = words + 3 * nw;
+  unsigned long long* totals = (unsigned long long*)(words + 4 * nw);
+  cudaMemsetAsync(totals, 0, sizeof(unsigned long long) * NTOT, s);
+  for (int64_t* q : {cnt_a, cnt_b}) cudaMemsetAsync(q + nrows, 0, sizeof(int64_t), s);
   const int64_t W = (A->ncols + P - 1) / P;  // columns per band
   const int* idx = (const int*)A->idx;
-  vrow_count_k<PtrT><<<grid, 256, 0, s>>>(nrows, ptr, idx, A->index_base, T, P, W, cnt_v, cnt_l, cnt_s, cnt_g,
-                                          cnt_ss, band_cnt);
-  cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, cnt_v, voff, nrows + 1, s);
+  vrow_count_k<PtrT><<<grid, 256, 0, s>>>(nrows, ptr, idx, A->index_base, T, P, W, cnt_a, cnt_b, totals);
+  cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, cnt_a, off_a, nw, s);
   if ((e = cudaMallocAsync(&cub_tmp, cub_bytes, s)) != cudaSuccess) return fail("alloc");
-  if ((e = cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, cnt_v, voff, nrows + 1, s)) != cudaSuccess)
-    return fail("scan");
-  const int64_t* cnts[5] = {cnt_v, cnt_l, cnt_s, cnt_g, cnt_ss};
-  int64_t* offs[5] = {voff, loff, soff, goff, ssoff};
-  for (int q = 1; q < 5; ++q)
-    if ((e = cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, cnts[q], offs[q], nrows + 1, s)) != cudaSuccess)
-      return fail("scan");
-  int64_t tot[5] = {0, 0, 0, 0, 0};
-  unsigned long long bcnt[VR_MAX_BANDS] = {};
-  for (int q = 0; q < 5; ++q)
-    cudaMemcpyAsync(&tot[q], offs[q] + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(bcnt, band_cnt, sizeof(bcnt), cudaMemcpyDeviceToHost, s);
+  if ((e = cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, cnt_a, off_a, nw, s)) != cudaSuccess) return fail("scan");
+  if ((e = cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, cnt_b, off_b, nw, s)) != cudaSuccess) return fail("scan");
+  int64_t tot_a = 0, tot_b = 0;
+  unsigned long long bcnt[VR_MAX_BANDS + 1] = {};
+  cudaMemcpyAsync(&tot_a, off_a + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(&tot_b, off_b + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(bcnt, totals, sizeof(bcnt), cudaMemcpyDeviceToHost, s);
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail("count");
-  const int64_t nv = tot[0], nl = tot[1], nseg = tot[2], nlong = tot[3], nss = tot[4];
+  const int64_t nv = vr_lo(tot_a), nl = vr_hi(tot_a), nseg = vr_lo(tot_b);
+  const int64_t nss = vr_hi(tot_b), nlong = (int64_t)bcnt[VR_MAX_BANDS];
   if (nv > INT32_MAX || nl > INT32_MAX) {
     release(false);
     return set_error(FGB_EUNSUPPORTED, "vrow schedule: too many virtual rows");
@@ -566,8 +568,8 @@ static int vrow_build_t(fgb_ctx* ctx, const fgb_sparse* A, int T, int P, VrowSch
   int32_t* ord = (int32_t*)(tmp + 2 * a256(nv));
   int32_t* ord2 = (int32_t*)(tmp + 2 * a256(nv) + a256(4 * nv));
   int4* unsorted = (int4*)(tmp + 2 * a256(nv) + 2 * a256(4 * nv));
-  vrow_fill_k<PtrT><<<grid, 256, 0, s>>>(nrows, ptr, idx, A->index_base, T, P, W, voff, loff, soff, goff, ssoff,
-                                         key, ord, unsorted, out->seg, out->lrow);
+  vrow_fill_k<PtrT><<<grid, 256, 0, s>>>(nrows, ptr, idx, A->index_base, T, P, W, off_a, off_b,
+                                         totals + VR_MAX_BANDS + 1, key, ord, unsorted, out->seg, out->lrow);
   const int end_bit = P > 1 ? 8 : 4;  // key: band << 5 | continues-C << 4 | length class
   b2 = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, b2, key, key2, ord, ord2, (int)nv, 0, end_bit, s);
