@@ -119,6 +119,14 @@ struct fgb_plan {
 
 namespace {
 
+// Whether the SpMM's operands suit the load-balanced CSR schedules.
+bool spmm_aligned(const fgb_plan* p) {
+  const fgb_plan_desc& d = p->d;
+  const int vn = d.dtype == FGB_F64 ? 2 : 4, esz = d.dtype == FGB_F64 ? 8 : 4;
+  return p->A.orient == FGB_CSR && !(d.flags & FGB_FINCH_ORDER) && d.k % vn == 0 && d.ld_in0 % vn == 0 &&
+         d.ld_out % vn == 0 && (uintptr_t)d.in0 % (vn * esz) == 0 && (uintptr_t)d.out % (vn * esz) == 0;
+}
+
 // Issues the operation with schedule `c` on stream s (no allocation, no sync).
 int issue(fgb_plan* p, const Choice& c, cudaStream_t s, bool plan_ready) {
   const fgb_plan_desc& d = p->d;
@@ -164,6 +172,9 @@ int issue(fgb_plan* p, const Choice& c, cudaStream_t s, bool plan_ready) {
         return spmm_merge(p->ctx, &p->A, d.in0, d.ld_in0, d.k, d.out, d.ld_out, d.dtype,
                           (d.flags & FGB_ACCUMULATE) ? 1 : 0, c.lanes, c.path, p->scratch,
                           p->scratch_bytes, s, plan_ready, nullptr, c.variant);
+      if (spmm_aligned(p))  // no item length: whole rows, equal shares per block
+        return spmm_auto(p->ctx, &p->A, d.in0, d.ld_in0, d.k, d.out, d.ld_out, d.dtype,
+                         (d.flags & FGB_ACCUMULATE) ? 1 : 0, s);
       return spmm_impl(p->ctx, &p->A, d.in0, d.ld_in0, d.k, d.out, d.ld_out, d.dtype, d.flags,
                        c.lanes, 0, s);
     case FGB_PLAN_SDDMM:
@@ -196,17 +207,15 @@ std::vector<Choice> candidates(const fgb_plan* p) {
     if (d.semiring == FGB_OR_AND && p->A.orient == FGB_CSC)
       out.push_back(Choice{0, 0});  // the warp-cooperative push over the true columns
   } else if (d.op == FGB_PLAN_SPMM) {
-    const int vn = d.dtype == FGB_F64 ? 2 : 4;
-    const bool merge = p->A.orient == FGB_CSR && !(d.flags & FGB_FINCH_ORDER) && d.k % vn == 0 &&
-                       d.ld_in0 % vn == 0 && d.ld_out % vn == 0 &&
-                       (uintptr_t)d.in0 % (vn * (d.dtype == FGB_F64 ? 8 : 4)) == 0 &&
-                       (uintptr_t)d.out % (vn * (d.dtype == FGB_F64 ? 8 : 4)) == 0;
-    if (!merge) {
+    if (!spmm_aligned(p)) {
       for (int l : {4, 8, 16, 32}) out.push_back(Choice{l, 0});
       return out;
     }
     for (int l : {8, 16, 32})
       for (int64_t path : {128, 256, 512, 1024}) out.push_back(Choice{l, path, 1, 0});
+    // spmm_auto: whole rows, equal shares per block; the lanes are those it takes
+    const int64_t need = d.k / (d.dtype == FGB_F64 ? 2 : 4);
+    out.push_back(Choice{need <= 4 ? 4 : need <= 8 ? 8 : need <= 16 ? 16 : 32, 0, 1, 0});
     if (d.dtype == FGB_F32)  // B rows staged by TMA into a shared-memory ring
       for (int64_t path : {256, 512, 1024, 2048}) out.push_back(Choice{32, path, 1, 1});
     if (d.dtype == FGB_F32 && p->A.val_t == FGB_F32 && p->A.nrows <= INT32_MAX)

@@ -22,21 +22,6 @@
 
 namespace fgb {
 
-// NB entries of a row, all of them stored: gathers first, then the updates in
-// storage order.  my_j/my_a: entry pb + lane of the group's current G entries.
-template <class T, int G, int V, int NB, int FM>
-__device__ __forceinline__ void pull_batch(VecT<T, V>& acc, int t, int my_j, T my_a, const T* __restrict__ Bc,
-                                           int64_t ldb, bool active, unsigned gmask, uint64_t pol) {
-  VecT<T, V> b[NB];
-#pragma unroll
-  for (int u = 0; u < NB; ++u) {
-    const int j = __shfl_sync(gmask, my_j, t + u, G);
-    if (active) b[u] = gather<T, V>(Bc + (int64_t)j * ldb, pol);
-  }
-#pragma unroll
-  for (int u = 0; u < NB; ++u) acc_step<T, V>(acc, __shfl_sync(gmask, my_a, t + u, G), b[u], FM);
-}
-
 // One launch = one column slab [c0, c0 + G*V) (clipped to nk) of every row.
 // A row's entries are taken in batches of 8, then 4, 2 and 1, so that no
 // gather or update slot is spent on entries the row does not have: FP64 is
@@ -189,7 +174,7 @@ static int default_lanes(int64_t nk, int vn, int64_t b_bytes) {
   return lanes;
 }
 
-// Default merge-path tuning: lanes enough for all of nk (up to 32, i.e.
+// Merge-path tuning where only a part of it is given: lanes enough for all of nk (up to 32, i.e.
 // whole 512-byte rows of fp32 B per gather), items of 256 path steps.
 // Narrower column slabs do not shrink B's L2 footprint on row-major B --
 // a 64-byte slice still occupies a whole 128-byte line -- and they re-read
@@ -221,6 +206,8 @@ static int run_typed(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t l
                         ((uintptr_t)B % (VN * sizeof(T)) == 0) &&
                         ((uintptr_t)C % (VN * sizeof(T)) == 0);
     if (!(flags & FGB_FINCH_ORDER) && vec_ok) {
+      if (variant == 0 && lanes <= 0 && path <= 0)
+        return spmm_auto(ctx, A, B, ldb, nk, C, ldc, sizeof(T) == 8 ? FGB_F64 : FGB_F32, accumulate, s);
       default_merge_tuning(A, nk, sizeof(T), &lanes, &path);
       return spmm_merge(ctx, A, B, ldb, nk, C, ldc, sizeof(T) == 8 ? FGB_F64 : FGB_F32,
                         accumulate, lanes, path, nullptr, 0, s, false, nullptr, variant);

@@ -73,6 +73,11 @@ int spmm_tma_items(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb
                    const int64_t* plan_k, int64_t* carry_row, void* carry, const int32_t* row_map,
                    int* err, cudaStream_t s);
 
+// Whole rows, equal shares of the rows and entries per block (spmm_auto.cu):
+// aligned CSR operands with no schedule given.
+int spmm_auto(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk, void* C, int64_t ldc,
+              int dtype, int accumulate, cudaStream_t s);
+
 template <class T, int V>
 struct VecT {
   T v[V];
@@ -136,6 +141,21 @@ template <class T, int V>
 __device__ __forceinline__ void acc_step(VecT<T, V>& acc, T a, const VecT<T, V>& b, int fm) {
 #pragma unroll
   for (int q = 0; q < V; ++q) acc.v[q] = Semi<SR_PT, T>::step(acc.v[q], a, b.v[q], fm);
+}
+
+// NB entries of a row, all of them stored: gathers first, then the updates in
+// storage order.  my_j/my_a: entry pb + lane of the group's current G entries.
+template <class T, int G, int V, int NB, int FM>
+__device__ __forceinline__ void pull_batch(VecT<T, V>& acc, int t, int my_j, T my_a, const T* __restrict__ Bc,
+                                           int64_t ldb, bool active, unsigned gmask, uint64_t pol) {
+  VecT<T, V> b[NB];
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    const int j = __shfl_sync(gmask, my_j, t + u, G);
+    if (active) b[u] = gather<T, V>(Bc + (int64_t)j * ldb, pol);
+  }
+#pragma unroll
+  for (int u = 0; u < NB; ++u) acc_step<T, V>(acc, __shfl_sync(gmask, my_a, t + u, G), b[u], FM);
 }
 
 }  // namespace fgb

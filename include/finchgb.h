@@ -260,7 +260,8 @@ FGB_API int fgb_spmv(fgb_ctx* ctx, int semiring, const fgb_sparse* A, const void
  * (ldb), C row-major (ldc).  F32 (A F32 or BF16 values, B/C F32) or F64.
  * Replaces `@einsum C[i,k] += A[i,j]*B[j,k]` = tensordot(A,B,(2,1))
  * (src/interface/lazy.jl:215-257,387-404).  CSR runs load-balanced
- * (merge-path items, deterministic carry fix-up); with FGB_FINCH_ORDER (or
+ * (whole rows in equal shares of rows and entries per block, or column slabs
+ * over virtual rows for a large B; deterministic); with FGB_FINCH_ORDER (or
  * an unaligned nk/ldb/ldc) each row is one running sum per column, j
  * ascending, bit-identical to Finch's nest.  CSC runs as a push with
  * atomics. */
@@ -283,7 +284,8 @@ FGB_API int fgb_spmm_semiring(fgb_ctx* ctx, int semiring, const fgb_sparse* A, c
  * entries) with groups of `lanes` lanes, each lane holding 4 (fp32) or 2
  * (fp64) consecutive columns; columns are processed in slabs of
  * lanes * vector-width, one launch per slab, so the gathered slab of B stays
- * L2-resident.  Zero fields take the defaults. */
+ * L2-resident.  Zero fields take the defaults; all zero, the library picks
+ * the schedule (fgb_spmm). */
 typedef struct fgb_spmm_tuning {
   int32_t lanes;   /* 2, 4, 8, 16 or 32 (variants 2 and 3: 2, 4 or 8) */
   int32_t variant; /* 0: B rows gathered into registers; 1: B rows staged into a

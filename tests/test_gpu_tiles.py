@@ -7,7 +7,7 @@ import oracle
 from finchgb import _lib as L
 from finchgb import device as dev
 from finchgb.workloads import SparseBuffers, _fibers_from_lengths, _ptr
-from helpers import abs_terms, assert_close, oracle_spmv, to_dev, to_host, upload
+from helpers import abs_terms, assert_close, bf16_bits, oracle_spmv, to_dev, to_host, upload
 
 pytestmark = pytest.mark.gpu
 
@@ -171,3 +171,33 @@ def test_ewise_tiles(gpu_lib, kind, dtype):
                 want = oracle.ewise_reduce(*args, a.val, b.ptr, b.idx, b.val)
                 scale = oracle.ewise_reduce(*args, np.abs(a.val), b.ptr, b.idx, np.abs(b.val))
                 assert_close(to_host(dev.ewise_reduce(dims, da, db)), want, scale, dtype)
+
+
+@pytest.mark.parametrize("dtype,bf16", [(np.float32, False), (np.float64, False), (np.float32, True)])
+@pytest.mark.parametrize("nk", [4, 12, 32, 60, 128, 132])
+def test_spmm_whole_rows(gpu_lib, dtype, bf16, nk):
+    """The default for aligned operands: groups of 4 to 32 lanes, lanes beyond
+    nk, a second slab of columns, rows at both sides of the length from which
+    the block folds a row, empty rows, blocks whose share lies inside one row;
+    within the bound, accumulating into strided rows too, and the same twice."""
+    rng = np.random.default_rng(nk)
+    lengths = rng.integers(0, 40, 3000)
+    lengths[100:140] = rng.integers(62, 68, 40)
+    lengths[[0, 7, 1500, 2999]] = (9000, 600, 65, 64)
+    lengths[2000:2300] = 0
+    r = csr_of_lengths(rng, lengths, 9500, dtype)
+    B = rng.standard_normal((9500, nk + 4)).astype(dtype)[:, :nk]
+    A, Bd = upload(r, as_bf16=bf16), to_dev(np.pad(B, ((0, 0), (0, 4))))[:, :nk]
+    Bc = np.ascontiguousarray(B)
+    val = bf16_bits(r.val) if bf16 else r.val
+    want = oracle.spmm_csr(3000, 9500, r.ptr, r.idx, val, Bc, bf16=bf16)
+    scale = oracle.spmm_csr(3000, 9500, r.ptr, r.idx, np.abs(r.val).astype(np.float64), np.abs(Bc).astype(np.float64))
+    C = to_host(dev.spmm(A, Bd))
+    assert_close(C, want, scale, dtype)
+    assert np.array_equal(C, to_host(dev.spmm(A, Bd)))
+    C0 = rng.standard_normal((3000, nk + 4)).astype(dtype)
+    Cd = to_dev(C0)
+    dev.spmm(A, Bd, Cd[:, :nk], flags=L.ACCUMULATE)
+    got = to_host(Cd)
+    assert_close(got[:, :nk], want.astype(np.float64) + C0[:, :nk], scale + np.abs(C0[:, :nk]), dtype)
+    assert np.array_equal(got[:, nk:], C0[:, nk:])
