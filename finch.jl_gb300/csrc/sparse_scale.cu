@@ -4,13 +4,14 @@
 //
 //     for j=_, i=_; if keep[k] != 0; out[i, j] = A[i, j] / by[l]; end; end
 //
-// Kept entries stay in A's order.  Each entry gets a keep flag; an
-// exclusive scan of the flags is its position in the result, and a fiber's
-// new ptr is the scan at the fiber's first entry, the prefix sum SparseList
-// assembly uses (src/tensors/levels/sparse_list_levels.jl:310-327).
+// Kept entries stay in A's order.  A block counts the kept entries of its run
+// and notes each one's place among them; a scan of the blocks' counts places
+// the runs, and a fiber's new ptr is the place of its first entry, the prefix
+// sum SparseList assembly uses (src/tensors/levels/
+// sparse_list_levels.jl:310-327).
 #include <cub/cub.cuh>
 
-#include "fgb_internal.cuh"
+#include "fiber_chunk.cuh"
 
 namespace fgb {
 
@@ -57,18 +58,6 @@ __global__ void count_fill_changed(int64_t n, const void* by, int by_t, int op,
   if ((threadIdx.x & 31) == 0 && mine) atomicAdd(count, mine);
 }
 
-// Fiber of entry p: the largest f with ptr[f] - base <= p.
-template <class PtrT>
-__device__ __forceinline__ int64_t fiber_of(const PtrT* __restrict__ ptr, int64_t nf, int base, int64_t p) {
-  int64_t lo = 0, hi = nf;
-  while (hi - lo > 1) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (ld_ptr(ptr, mid) - base <= p) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
 struct ScaleArgs {
   int64_t nnz, nf;
   int base, csc, op, by_axis, by_t, keep_axis, keep_t, val_t, out_t;
@@ -76,23 +65,56 @@ struct ScaleArgs {
   const void *val, *by, *keep;
 };
 
-// flag[p] = 1 when entry p is kept (flag[nnz] = 0 closes the scan).
+// local[p] = kept entries of the block's run before entry p, times 2, plus 1
+// where entry p is kept; count[b] = kept entries of run b (count[runs] = 0
+// closes the scan).
 template <class PtrT>
-__global__ void scale_flags(ScaleArgs a, const PtrT* __restrict__ ptr, int64_t* __restrict__ flag) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p <= a.nnz;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    if (p == a.nnz) {
-      flag[p] = 0;
-      continue;
+__global__ void __launch_bounds__(FC_THREADS) scale_flags(ScaleArgs a, const PtrT* __restrict__ ptr,
+                                                          int32_t* __restrict__ local,
+                                                          int64_t* __restrict__ count) {
+  constexpr int ROUNDS = FC_ENTRIES / FC_THREADS, WARPS = FC_THREADS / 32;
+  static_assert(ROUNDS * WARPS == 64, "two words per lane below");
+  __shared__ int s_starts[FC_FIBERS];
+  __shared__ int s_before[ROUNDS * WARPS];
+  const int64_t p0 = (int64_t)blockIdx.x * FC_ENTRIES;
+  const int n = a.nnz - p0 < FC_ENTRIES ? (int)(a.nnz - p0) : FC_ENTRIES;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned kept = 0;  // bit u: entry u * FC_THREADS + tid
+  int before[ROUNDS];
+  const FiberChunk<PtrT> fibers(ptr, a.nf, a.base, p0, n, s_starts);
+#pragma unroll
+  for (int u = 0; u < ROUNDS; ++u) {
+    const int e = u * FC_THREADS + tid;
+    bool keep = e < n;
+    if (keep && a.keep) {
+      const int64_t c = (int64_t)__ldg(a.idx + p0 + e) - a.base;
+      const bool is_fiber = (a.keep_axis == FGB_AXIS_COL) == (a.csc != 0);
+      keep = nonzero_at(a.keep, a.keep_t, is_fiber ? fibers.of(e) : c);
     }
-    if (!a.keep) {
-      flag[p] = 1;
-      continue;
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    kept |= (keep ? 1u : 0u) << u;
+    before[u] = __popc(m & ((1u << lane) - 1));
+    if (lane == 0) s_before[u * WARPS + warp] = __popc(m);
+  }
+  __syncthreads();
+  if (warp == 0) {  // exclusive scan of the 64 counts
+    const int x = s_before[2 * lane], y = s_before[2 * lane + 1];
+    int incl = x + y;
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, m);
+      if (lane >= m) incl += t;
     }
-    const int64_t f = fiber_of(ptr, a.nf, a.base, p);
-    const int64_t c = (int64_t)__ldg(a.idx + p) - a.base;
-    const int64_t i = a.csc ? c : f, j = a.csc ? f : c;
-    flag[p] = nonzero_at(a.keep, a.keep_t, a.keep_axis == FGB_AXIS_ROW ? i : j) ? 1 : 0;
+    s_before[2 * lane] = incl - x - y;
+    s_before[2 * lane + 1] = incl - y;
+    if (lane == 31) count[blockIdx.x] = incl;
+  }
+  if (blockIdx.x == gridDim.x - 1 && tid == 0) count[gridDim.x] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < ROUNDS; ++u) {
+    const int e = u * FC_THREADS + tid;
+    if (e < n) local[p0 + e] = (s_before[u * WARPS + warp] + before[u]) << 1 | ((kept >> u) & 1);
   }
 }
 
@@ -102,17 +124,25 @@ __device__ __forceinline__ T combine(T v, T b, int op) {
 }
 
 template <class PtrT>
-__global__ void scale_write(ScaleArgs a, const PtrT* __restrict__ ptr, const int64_t* __restrict__ flag,
-                            const int64_t* __restrict__ pos, int32_t* __restrict__ out_idx,
-                            void* __restrict__ out_val, bool in_f32) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.nnz;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    if (!flag[p]) continue;
-    const int64_t f = fiber_of(ptr, a.nf, a.base, p);
+__global__ void __launch_bounds__(FC_THREADS) scale_write(ScaleArgs a, const PtrT* __restrict__ ptr,
+                                                          const int32_t* __restrict__ local,
+                                                          const int64_t* __restrict__ run_pos,
+                                                          int32_t* __restrict__ out_idx,
+                                                          void* __restrict__ out_val, bool in_f32) {
+  __shared__ int s_starts[FC_FIBERS];
+  const int64_t p0 = (int64_t)blockIdx.x * FC_ENTRIES;
+  const int n = a.nnz - p0 < FC_ENTRIES ? (int)(a.nnz - p0) : FC_ENTRIES;
+  const bool by_fiber = (a.by_axis == FGB_AXIS_COL) == (a.csc != 0);
+  const FiberChunk<PtrT> fibers(ptr, a.nf, a.base, p0, n, s_starts);
+  const int64_t q0 = run_pos[blockIdx.x];
+#pragma unroll 2
+  for (int e = threadIdx.x; e < n; e += FC_THREADS) {
+    const int64_t p = p0 + e;
+    const int32_t w = local[p];
+    if (!(w & 1)) continue;
     const int c = __ldg(a.idx + p) - a.base;
-    const int64_t i = a.csc ? c : f, j = a.csc ? f : c;
-    const int64_t l = a.by_axis == FGB_AXIS_ROW ? i : j;
-    const int64_t q = pos[p];
+    const int64_t l = by_fiber ? fibers.of(e) : c;
+    const int64_t q = q0 + (w >> 1);
     out_idx[q] = c;
     if (in_f32) {  // Julia's promotion: F32 with F32 or an integer stays F32
       const float r = combine(load_as<float>(a.val, a.val_t, p), load_as<float>(a.by, a.by_t, l), a.op);
@@ -126,12 +156,15 @@ __global__ void scale_write(ScaleArgs a, const PtrT* __restrict__ ptr, const int
   }
 }
 
-// out_ptr[f] = pos[ptr[f] - base] for f <= nf: pos[nnz] is the kept count.
+// out_ptr[f] = the place of fiber f's first entry, for f <= nf.
 template <class PtrT>
-__global__ void scale_ptr(int64_t nf, const PtrT* __restrict__ ptr, int base, const int64_t* __restrict__ pos,
+__global__ void scale_ptr(int64_t nnz, int64_t nf, const PtrT* __restrict__ ptr, int base,
+                          const int32_t* __restrict__ local, const int64_t* __restrict__ run_pos,
                           int64_t* __restrict__ out_ptr) {
-  for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f <= nf; f += (int64_t)gridDim.x * blockDim.x)
-    out_ptr[f] = pos[ld_ptr(ptr, f) - base];
+  for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f <= nf; f += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = ld_ptr(ptr, f) - base;
+    out_ptr[f] = p < nnz ? run_pos[p / FC_ENTRIES] + (local[p] >> 1) : run_pos[(nnz + FC_ENTRIES - 1) / FC_ENTRIES];
+  }
 }
 
 static bool value_type_ok(int t) {
@@ -143,29 +176,34 @@ static int sparse_scale_typed(fgb_ctx* ctx, const fgb_sparse* A, const ScaleArgs
                               int32_t* out_idx, void* out_val, int64_t* out_nnz, bool in_f32,
                               cudaStream_t s) {
   const PtrT* ptr = (const PtrT*)A->ptr;
-  int64_t *flag = nullptr, *pos = nullptr;
+  const int64_t runs = fc_blocks(a.nnz);
+  char* mem = nullptr;  // places within the runs, the runs' counts and their scan
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flag, pos, a.nnz + 1, s);
+  cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (int64_t*)nullptr, (int64_t*)nullptr, runs + 1, s);
+  const size_t head = (sizeof(int32_t) * a.nnz + 255) & ~size_t(255);
   int rc = FGB_OK;
-  cudaError_t e = cudaMallocAsync((void**)&flag, sizeof(int64_t) * (a.nnz + 1) * 2, s);
+  cudaError_t e = cudaMallocAsync((void**)&mem, head + sizeof(int64_t) * (runs + 1) * 2, s);
   if (e == cudaSuccess) e = cudaMallocAsync(&tmp, tmp_bytes, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(mem + head, 0, sizeof(int64_t) * (runs + 1), s);
   if (e != cudaSuccess) {
     rc = set_error(FGB_ENOMEM, "fgb_sparse_scale: scratch allocation failed: %s", cudaGetErrorString(e));
   } else {
-    pos = flag + (a.nnz + 1);
-    const int grid = grid_for(a.nnz + 1, 256, ctx->num_sms, 8);
-    scale_flags<PtrT><<<grid, 256, 0, s>>>(a, ptr, flag);
-    cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flag, pos, a.nnz + 1, s);
-    scale_write<PtrT><<<grid, 256, 0, s>>>(a, ptr, flag, pos, out_idx, out_val, in_f32);
-    scale_ptr<PtrT><<<grid_for(a.nf + 1, 256, ctx->num_sms, 8), 256, 0, s>>>(a.nf, ptr, a.base, pos, out_ptr);
+    int32_t* local = (int32_t*)mem;
+    int64_t *count = (int64_t*)(mem + head), *pos = count + (runs + 1);
+    if (runs > 0) scale_flags<PtrT><<<(unsigned)runs, FC_THREADS, 0, s>>>(a, ptr, local, count);
+    cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, count, pos, runs + 1, s);
+    if (runs > 0)
+      scale_write<PtrT><<<(unsigned)runs, FC_THREADS, 0, s>>>(a, ptr, local, pos, out_idx, out_val, in_f32);
+    scale_ptr<PtrT><<<grid_for(a.nf + 1, 256, ctx->num_sms, 8), 256, 0, s>>>(a.nnz, a.nf, ptr, a.base, local, pos,
+                                                                           out_ptr);
     rc = check_launch("fgb_sparse_scale");
     if (rc == FGB_OK) {
-      e = cudaMemcpyAsync(out_nnz, pos + a.nnz, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+      e = cudaMemcpyAsync(out_nnz, pos + runs, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
       if (e != cudaSuccess) rc = set_error(FGB_ECUDA, "fgb_sparse_scale: %s", cudaGetErrorString(e));
     }
   }
-  if (flag) cudaFreeAsync(flag, s);
+  if (mem) cudaFreeAsync(mem, s);
   if (tmp) cudaFreeAsync(tmp, s);
   cudaError_t se = cudaStreamSynchronize(s);
   if (rc == FGB_OK && se != cudaSuccess) rc = set_error(FGB_ECUDA, "fgb_sparse_scale: %s", cudaGetErrorString(se));

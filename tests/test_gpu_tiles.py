@@ -2,6 +2,7 @@
 at the sizes where a cut can go wrong, against the oracle."""
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from finchgb import _lib as L
@@ -201,3 +202,46 @@ def test_spmm_whole_rows(gpu_lib, dtype, bf16, nk):
     got = to_host(Cd)
     assert_close(got[:, :nk], want.astype(np.float64) + C0[:, :nk], scale + np.abs(C0[:, :nk]), dtype)
     assert np.array_equal(got[:, nk:], C0[:, nk:])
+
+
+@pytest.mark.parametrize("kind", ["dense", "hollow", "long"])
+@pytest.mark.parametrize("val", ["f64", "i32", "bf16", "bool", "pattern"])
+def test_transpose_and_scale_runs(gpu_lib, kind, val):
+    """Kernels that find the fiber of every entry of a run of 2,048: runs with
+    few fibers, with more than their shared memory holds (mostly empty), and
+    inside one fiber; first and last fibers empty, a last run not full.
+    Transposes and masked scalings equal numpy's, every payload width."""
+    rng = np.random.default_rng(len(kind))
+    if kind == "dense":
+        lengths = rng.integers(0, 30, 900)
+    elif kind == "hollow":
+        lengths = (rng.random(60_000) < 0.1).astype(np.int64)
+    else:
+        lengths = np.array([0, 0, 5000, 0, 1, 2047, 0])
+    lengths[[0, -1]] = 0
+    n = 5200
+    b = csr_of_lengths(rng, lengths, n, np.float64)
+    f = np.repeat(np.arange(lengths.size), lengths)
+    t = {"f64": torch.float64, "i32": torch.int32, "bf16": torch.bfloat16, "bool": torch.uint8, "pattern": None}[val]
+    A = upload(b)
+    if t is None:
+        A = dev.DeviceSparse(A.nrows, A.ncols, A.ptr, A.idx, None, "csr", 1)
+        v = np.ones(b.nnz)
+    else:
+        A.val = (A.val * 3).to(torch.int64).clamp(0, 1).to(t) if t == torch.uint8 else (A.val * 3).to(t)
+        v = A.val.double().cpu().numpy()
+    T = A.transposed_storage()
+    order = np.lexsort((f, b.idx))
+    assert np.array_equal(T.idx.cpu().numpy(), f[order])
+    assert np.array_equal(np.diff(T.ptr.cpu().numpy()), np.bincount(b.idx - 1, minlength=n))
+    if t is not None:
+        assert np.array_equal(T.val.double().cpu().numpy(), v[order])
+    if val == "bf16":
+        return
+    keep = rng.integers(0, 3, n).astype(np.float64)
+    by = rng.integers(1, 9, lengths.size).astype(np.float64)
+    S, changed = dev.sparse_scale(A, to_dev(by), L.AXIS_ROW, to_dev(keep), L.AXIS_COL, L.MAP_MUL)
+    kept = keep[b.idx - 1] != 0
+    assert changed == 0 and np.array_equal(S.idx.cpu().numpy(), b.idx[kept] - 1)
+    assert np.array_equal(S.val.cpu().numpy(), (v * by[f])[kept])
+    assert np.array_equal(np.diff(S.ptr.cpu().numpy()), np.bincount(f[kept], minlength=lengths.size))
