@@ -247,4 +247,6 @@ def check(status: int, what: str = "") -> None:
 
 def call(name: str, *args) -> None:
     """Calls an entry point and raises FinchGBError on a non-zero status."""
-    check(getattr(load(), name)(*args), name)
+    status = getattr(_lib or load(), name)(*args)
+    if status != OK:
+        check(status, name)

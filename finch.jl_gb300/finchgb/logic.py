@@ -105,6 +105,8 @@ def indices_of(n: Node) -> tuple:
 def flatten(n: Node) -> Node:
     """Flattens nested MapJoins of the same associative operator."""
     if isinstance(n, MapJoin):
+        if all(isinstance(a, (Access, Literal)) for a in n.args):
+            return n  # nothing below it to flatten
         args = []
         for a in map(flatten, n.args):
             if isinstance(a, MapJoin) and a.op == n.op and n.op in ASSOCIATIVE:
@@ -190,13 +192,22 @@ class EinsumPlan:
         return Reorder(body, self.out_idxs)
 
 
-def parse_einsum(stmt: str, tensors: dict, init=None) -> EinsumPlan:
-    """Parses `out[i,...] <op>= expr` (src/interface/einsum.jl:136-201)."""
+@functools.lru_cache(maxsize=512)
+def _statement(stmt: str):
+    """The parts of a statement's text, matched once per text."""
     m = _LHS.match(stmt)
     if not m:
-        raise SyntaxError(f"einsum: cannot parse {stmt!r}")
+        return None
     name, idxs, assign, custom, rhs = m.groups()
-    out_idxs = tuple(s.strip() for s in idxs.split(",") if s.strip())
+    return name, tuple(s.strip() for s in idxs.split(",") if s.strip()), assign, custom, rhs
+
+
+def parse_einsum(stmt: str, tensors: dict, init=None) -> EinsumPlan:
+    """Parses `out[i,...] <op>= expr` (src/interface/einsum.jl:136-201)."""
+    parts = _statement(stmt)
+    if parts is None:
+        raise SyntaxError(f"einsum: cannot parse {stmt!r}")
+    name, out_idxs, assign, custom, rhs = parts
     if custom and (custom == "overwrite" or custom.startswith("initwrite(")):
         # overwrite(a, b) = b and initwrite(z)(a, b) = b (src/util/special_
         # functions.jl): assignments, not reductions -- the `=` form, with

@@ -20,6 +20,7 @@ tensors then stay resident across calls.
 """
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass
 
 import numpy as np
@@ -750,15 +751,15 @@ def transfer(device, t):
 
     Sparse levels are narrowed to int32 idx once; dense levels are copied
     row-major.  Returns the same tensor object, now resident."""
-    import torch
-
-    from . import device as dev
-
     if isinstance(t, SwizzleArray):
         transfer(device, t.body)
         return t
     if t.on_device:
         return t
+    import torch
+
+    from . import device as dev
+
     idx = device.index if isinstance(device, GPU) else int(device)
     if t.kind == "dense1" and t.dtype.names:  # tuple elements: one device array per component
         d = torch.device("cuda", idx)
@@ -829,9 +830,15 @@ def set_fill_value(t, fill):
     return SwizzleArray(out, t.dims) if isinstance(t, SwizzleArray) else out
 
 
+@functools.lru_cache(maxsize=None)
+def _numpy_of(dtype) -> np.dtype:
+    """The element type of a device array: torch's, one-byte Bools."""
+    return np.dtype(str(dtype).replace("torch.", "").replace("uint8", "bool"))
+
+
 def dense_from_device(x, fill_value=0.0) -> Tensor:
     """Wraps a device array (torch) as a Dense tensor resident in HBM."""
-    dt = np.dtype(str(x.dtype).replace("torch.", "").replace("uint8", "bool"))
+    dt = _numpy_of(x.dtype)
     fmt = Dense(Element(fill_value, dt)) if x.dim() == 1 else Dense(Dense(Element(fill_value, dt)))
     t = Tensor.__new__(Tensor)
     t.fmt, t.kind = fmt, ("dense1" if x.dim() == 1 else "dense2")
