@@ -53,9 +53,12 @@ constexpr int CG_ILP = 4;  // elements per thread in flight in the streaming upd
 // elements in flight (up to 64 registers): few partials, one load per thread
 // in each block's fold of the previous kernel's partials.
 constexpr int CG_UPD_THREADS = 1024;
-// Rows in flight per thread in the pair SpMVs (32-bit index build): 4
-// measured slower than 2 (BF16 pair CG 0.694 against 0.637 s).
-constexpr int CG_PAIR_ROWS = 2;
+// The SpMVs give a thread one row at a time: with 64 warps an SM the rows in
+// flight suffice, and a second row of its own costs a warp the longer of the
+// two and more instructions per entry.  2048^2 Poisson solve, two rows -> one:
+// FP64 816 -> 747 ms, BF16 SpMV pairs 764 -> 711, BF16 pairs 636 -> 608 (four
+// rows 694).  Values widened to FP64 or summed in FP32 keep two (1001 against
+// 1022 ms, 785 against 780).
 
 // The iteration kernels are chained by programmatic dependent launch: each
 // lets the next one launch as soon as it starts, and waits for the previous
@@ -176,26 +179,37 @@ __global__ void __launch_bounds__(CG_THREADS) cg_spmv_dot(
       return __fma_rn((double)cg_val(val, k), __ldg(p + j), acc);
   };
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  // two rows (i, i + stride) per thread in flight; rows and their products
-  // in the plain loop's order, so q and the partial are bit-identical
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += 2 * stride) {
-    const int64_t i2 = i + stride;
-    const bool two = i2 < n;
-    const int64_t a0 = ld_ptr(ptr, i) - base, a1 = ld_ptr(ptr, i + 1) - base;
-    const int64_t b0 = two ? ld_ptr(ptr, i2) - base : 0, b1 = two ? ld_ptr(ptr, i2 + 1) - base : 0;
-    ACC acc_a = ACC(0), acc_b = ACC(0);
-    const int64_t la = a1 - a0, lb = b1 - b0;
-    for (int64_t t = 0; t < (la > lb ? la : lb); ++t) {
-      if (t < la) acc_a = term(a0 + t, i, acc_a);
-      if (t < lb) acc_b = term(b0 + t, i2, acc_b);
+  if constexpr (sizeof(VT) == 8) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
+      const int64_t a0 = ld_ptr(ptr, i) - base, a1 = ld_ptr(ptr, i + 1) - base;
+      ACC acc = ACC(0);
+      for (int64_t k = a0; k < a1; ++k) acc = term(k, i, acc);
+      const double qv = (double)acc;
+      q[i] = qv;
+      dot = __fma_rn(__ldg(p + i), qv, dot);
     }
-    const double qa = (double)acc_a;
-    q[i] = qa;
-    dot = __fma_rn(__ldg(p + i), qa, dot);
-    if (two) {
-      const double qb = (double)acc_b;
-      q[i2] = qb;
-      dot = __fma_rn(__ldg(p + i2), qb, dot);
+  } else {
+    // two rows (i, i + stride) per thread in flight; rows and their products
+    // in the plain loop's order, so q and the partial are bit-identical
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += 2 * stride) {
+      const int64_t i2 = i + stride;
+      const bool two = i2 < n;
+      const int64_t a0 = ld_ptr(ptr, i) - base, a1 = ld_ptr(ptr, i + 1) - base;
+      const int64_t b0 = two ? ld_ptr(ptr, i2) - base : 0, b1 = two ? ld_ptr(ptr, i2 + 1) - base : 0;
+      ACC acc_a = ACC(0), acc_b = ACC(0);
+      const int64_t la = a1 - a0, lb = b1 - b0;
+      for (int64_t t = 0; t < (la > lb ? la : lb); ++t) {
+        if (t < la) acc_a = term(a0 + t, i, acc_a);
+        if (t < lb) acc_b = term(b0 + t, i2, acc_b);
+      }
+      const double qa = (double)acc_a;
+      q[i] = qa;
+      dot = __fma_rn(__ldg(p + i), qa, dot);
+      if (two) {
+        const double qb = (double)acc_b;
+        q[i2] = qb;
+        dot = __fma_rn(__ldg(p + i2), qb, dot);
+      }
     }
   }
   dot = cg_block_sum(dot, sh);
@@ -220,7 +234,7 @@ __device__ __forceinline__ void ff_row_term(float& h, float& l, float a, float2 
 // the partial leaves the block as one FP64 number.  IT: the row, entry and
 // column arithmetic (int32 when rows and entries stay below 2^31, which
 // halves the integer instructions per entry).
-template <class VT, class PtrT, class IX, class IT, int R>
+template <class VT, class PtrT, class IX, class IT>
 __global__ void __launch_bounds__(CG_THREADS) cgp_spmv_dot(
     int64_t n64, const PtrT* __restrict__ ptr, const IX* __restrict__ idx, const VT* __restrict__ val,
     int base, const float2* __restrict__ p, float2* __restrict__ q, double* __restrict__ part) {
@@ -233,41 +247,14 @@ __global__ void __launch_bounds__(CG_THREADS) cgp_spmv_dot(
     if constexpr (sizeof(IX) == 2) return row + (IT)__ldg(idx + k);
     else return (IT)__ldg(idx + k) - (IT)base;
   };
-  // R rows (i, i + stride, ...) per thread in flight; the rows, and each
-  // row's products, in the plain loop's order, so q and the partial do not
-  // depend on R
-  for (IT i = (IT)blockIdx.x * (IT)blockDim.x + (IT)threadIdx.x; i < n; i += R * stride) {
-    IT s0[R], len[R];
-    IT lmax = 0;
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-      const IT row = i + (IT)u * stride;
-      s0[u] = 0;
-      len[u] = 0;
-      if (row < n) {
-        s0[u] = (IT)(ld_ptr(ptr, row) - base);
-        len[u] = (IT)(ld_ptr(ptr, row + 1) - base) - s0[u];
-      }
-      lmax = len[u] > lmax ? len[u] : lmax;
-    }
-    float h[R], l[R];
-#pragma unroll
-    for (int u = 0; u < R; ++u) h[u] = l[u] = 0.f;
-    for (IT t = 0; t < lmax; ++t) {
-#pragma unroll
-      for (int u = 0; u < R; ++u)
-        if (t < len[u])
-          ff_row_term(h[u], l[u], cg_val(val, s0[u] + t), __ldg(p + col(s0[u] + t, i + (IT)u * stride)));
-    }
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-      const IT row = i + (IT)u * stride;
-      if (row < n) {
-        const float2 acc = two_sum(h[u], l[u]);  // l may exceed h after cancellation
-        q[row] = acc;
-        dot = ff_add(dot, ff_mul(__ldg(p + row), acc));
-      }
-    }
+  for (IT i = (IT)blockIdx.x * (IT)blockDim.x + (IT)threadIdx.x; i < n; i += stride) {
+    const IT s0 = (IT)(ld_ptr(ptr, i) - base), s1 = (IT)(ld_ptr(ptr, i + 1) - base);
+    float h = 0.f, l = 0.f;
+    for (IT t = s0; t < s1; ++t)
+      ff_row_term(h, l, cg_val(val, t), __ldg(p + col(t, i)));
+    const float2 acc = two_sum(h, l);  // l may exceed h after cancellation
+    q[i] = acc;
+    dot = ff_add(dot, ff_mul(__ldg(p + i), acc));
   }
   dot = ff_block_sum(dot, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = ff_to_double(dot);
@@ -299,7 +286,7 @@ __device__ __forceinline__ float2 split_f64(double v) {
 // The SpMV of the pair-sum SpMV mode: FP64 p split into pairs as it is
 // gathered, each row summed as a pair (ff_row_term), q and the p.q partial
 // in FP64 -- the vectors, dots and updates stay FP64.
-template <class VT, class PtrT, class IX, class IT, int R>
+template <class VT, class PtrT, class IX, class IT>
 __global__ void __launch_bounds__(CG_THREADS) cgs_spmv_dot(
     int64_t n64, const PtrT* __restrict__ ptr, const IX* __restrict__ idx, const VT* __restrict__ val,
     int base, const double* __restrict__ p, double* __restrict__ q, double* __restrict__ part) {
@@ -312,38 +299,14 @@ __global__ void __launch_bounds__(CG_THREADS) cgs_spmv_dot(
     if constexpr (sizeof(IX) == 2) return row + (IT)__ldg(idx + k);
     else return (IT)__ldg(idx + k) - (IT)base;
   };
-  for (IT i = (IT)blockIdx.x * (IT)blockDim.x + (IT)threadIdx.x; i < n; i += R * stride) {
-    IT s0[R], len[R];
-    IT lmax = 0;
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-      const IT row = i + (IT)u * stride;
-      s0[u] = 0;
-      len[u] = 0;
-      if (row < n) {
-        s0[u] = (IT)(ld_ptr(ptr, row) - base);
-        len[u] = (IT)(ld_ptr(ptr, row + 1) - base) - s0[u];
-      }
-      lmax = len[u] > lmax ? len[u] : lmax;
-    }
-    float h[R], l[R];
-#pragma unroll
-    for (int u = 0; u < R; ++u) h[u] = l[u] = 0.f;
-    for (IT t = 0; t < lmax; ++t) {
-#pragma unroll
-      for (int u = 0; u < R; ++u)
-        if (t < len[u])
-          ff_row_term(h[u], l[u], cg_val(val, s0[u] + t), split_f64(__ldg(p + col(s0[u] + t, i + (IT)u * stride))));
-    }
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-      const IT row = i + (IT)u * stride;
-      if (row < n) {
-        const double qv = ff_to_double(two_sum(h[u], l[u]));
-        q[row] = qv;
-        dot = __fma_rn(__ldg(p + row), qv, dot);
-      }
-    }
+  for (IT i = (IT)blockIdx.x * (IT)blockDim.x + (IT)threadIdx.x; i < n; i += stride) {
+    const IT s0 = (IT)(ld_ptr(ptr, i) - base), s1 = (IT)(ld_ptr(ptr, i + 1) - base);
+    float h = 0.f, l = 0.f;
+    for (IT t = s0; t < s1; ++t)
+      ff_row_term(h, l, cg_val(val, t), split_f64(__ldg(p + col(t, i))));
+    const double qv = ff_to_double(two_sum(h, l));
+    q[i] = qv;
+    dot = __fma_rn(__ldg(p + i), qv, dot);
   }
   dot = cg_block_sum(dot, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = dot;
@@ -639,7 +602,7 @@ struct CgBuffers {
 enum CgMode { CG_F32_SUMS = 0, CG_F64_SUMS = 1, CG_PAIR_SUMS = 2, CG_SPMV_PAIR = 3 };
 
 // The SpMV's own grid: at most `grid` blocks and no more than fit the SMs at
-// once (its two rows per thread take more registers than the updates).
+// once.
 template <class K>
 static int occupancy_grid(K kernel, int grid, int sms) {
   int o = 0;
@@ -664,38 +627,38 @@ static int spmv_dot_t(const fgb_sparse* A, const IX* ix, int mode, int grid, int
     return g;
   } else {
     if (mode == CG_PAIR_SUMS) {
-      // 32-bit index arithmetic while rows (two per thread, a grid-stride
-      // apart) and entries stay below 2^31
-      const bool i32 = n + (int64_t)CG_PAIR_ROWS * grid * CG_THREADS < INT32_MAX && A->nnz < INT32_MAX;
+      // 32-bit index arithmetic while rows (one grid-stride beyond the last
+      // too) and entries stay below 2^31
+      const bool i32 = n + (int64_t)grid * CG_THREADS < INT32_MAX && A->nnz < INT32_MAX;
       if (i32) {
-        static const int g0 = occupancy_grid(cgp_spmv_dot<VT, PtrT, IX, int32_t, CG_PAIR_ROWS>, 1 << 30, 1);
+        static const int g0 = occupancy_grid(cgp_spmv_dot<VT, PtrT, IX, int32_t>, 1 << 30, 1);
         const int g = std::max(1, std::min(grid, g0 * sms));
         if (launch)
-          cg_launch(cgp_spmv_dot<VT, PtrT, IX, int32_t, CG_PAIR_ROWS>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
+          cg_launch(cgp_spmv_dot<VT, PtrT, IX, int32_t>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
                     (const float2*)b.p2, b.q2, b.part_a);
         return g;
       }
-      static const int g0 = occupancy_grid(cgp_spmv_dot<VT, PtrT, IX, int64_t, 2>, 1 << 30, 1);
+      static const int g0 = occupancy_grid(cgp_spmv_dot<VT, PtrT, IX, int64_t>, 1 << 30, 1);
       const int g = std::max(1, std::min(grid, g0 * sms));
       if (launch)
-        cg_launch(cgp_spmv_dot<VT, PtrT, IX, int64_t, 2>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
+        cg_launch(cgp_spmv_dot<VT, PtrT, IX, int64_t>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
                   (const float2*)b.p2, b.q2, b.part_a);
       return g;
     }
     if (mode == CG_SPMV_PAIR) {
-      const bool i32 = n + (int64_t)CG_PAIR_ROWS * grid * CG_THREADS < INT32_MAX && A->nnz < INT32_MAX;
+      const bool i32 = n + (int64_t)grid * CG_THREADS < INT32_MAX && A->nnz < INT32_MAX;
       if (i32) {
-        static const int g0 = occupancy_grid(cgs_spmv_dot<VT, PtrT, IX, int32_t, CG_PAIR_ROWS>, 1 << 30, 1);
+        static const int g0 = occupancy_grid(cgs_spmv_dot<VT, PtrT, IX, int32_t>, 1 << 30, 1);
         const int g = std::max(1, std::min(grid, g0 * sms));
         if (launch)
-          cg_launch(cgs_spmv_dot<VT, PtrT, IX, int32_t, CG_PAIR_ROWS>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
+          cg_launch(cgs_spmv_dot<VT, PtrT, IX, int32_t>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
                     (const double*)b.p, b.q, b.part_a);
         return g;
       }
-      static const int g0 = occupancy_grid(cgs_spmv_dot<VT, PtrT, IX, int64_t, 2>, 1 << 30, 1);
+      static const int g0 = occupancy_grid(cgs_spmv_dot<VT, PtrT, IX, int64_t>, 1 << 30, 1);
       const int g = std::max(1, std::min(grid, g0 * sms));
       if (launch)
-        cg_launch(cgs_spmv_dot<VT, PtrT, IX, int64_t, 2>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
+        cg_launch(cgs_spmv_dot<VT, PtrT, IX, int64_t>, g, CG_THREADS, s, pdl, n, ptr, ix, val, base,
                   (const double*)b.p, b.q, b.part_a);
       return g;
     }
