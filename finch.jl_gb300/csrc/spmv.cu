@@ -76,7 +76,12 @@ __global__ void __launch_bounds__(256) spmv_csr_pull(int64_t nrows, const PtrT* 
 // entries by its own lane, or, where the 32 rows average SPMV_MEAN4 entries,
 // by 4 lanes (a lane's loads are uncoalesced: long enough rows pay for the
 // two shuffles); a longer row by the whole warp, one of more than SPMV_BLOCK
-// entries by way of the list.
+// entries by way of the list.  Where the 32 rows average fewer than
+// SPMV_SPARSE entries of 8 bytes, rows over SPMV_SPARSE_LONG count as long:
+// the few lanes that had one kept the warp, and FP64 its pipe, busy for as
+// many steps (Zipf 1M x 16, FP64, 153 -> 139 us; 4M x 2 118 -> 103).  For
+// 4-byte values it gains 2-7 % there, but the 32-register build then spills
+// and the 4M-node graph loses 5 %.
 //
 // When a block's warps are done they share its list, the longest rows by the
 // whole block; a full list is no loss but in speed.  `ordered`
@@ -86,12 +91,11 @@ __global__ void __launch_bounds__(256) spmv_csr_pull(int64_t nrows, const PtrT* 
 // Bound: the gathers of x (one L1 tag a clock per SM), FP64 folds also by the
 // FP64 pipe.  GB300, per call, against rows of at most 32 entries on a lane
 // and longer ones by their warp in turn, with the contraction chosen at run
-// time: Zipf 1M x 16 FP64 286 -> 145 us with three operands in rotation, 85 in
-// a replay; uniform 4M x 8: FP64 360 -> 183, FP32 156 -> 142, Int32 min-plus
+// time: Zipf 1M x 16 FP64 283 -> 145 us with three operands in rotation; uniform 4M x 8: FP64 360 -> 183, FP32 156 -> 142, Int32 min-plus
 // 149 -> 140.  Staging tiles of entries in shared memory (coalesced, every
 // row folded from there) measured 298 (FP64) and 184 (FP32) on the uniform
 // rows, and equal shares alone 194 and 162.
-constexpr int SPMV_LONG = 32;
+constexpr int SPMV_LONG = 32, SPMV_SPARSE_LONG = 16, SPMV_SPARSE = 6;
 constexpr int SPMV_BLOCK = 2048;  // a warp alone takes 8 us for one
 constexpr int SPMV_LIST = 64;  // rows a block can leave to the end
 constexpr int SPMV_MEAN4 = 14;
@@ -225,9 +229,11 @@ __global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int
         n = ld_ptr(ptr, row + 1) - base - p0;
         if (p0 + base - f0 + row >= end) n = -1;
       }
-      const bool is_long = n > SPMV_LONG;
+      const int filled = sizeof(A) == 8 || !ordered  // entries in rows of at most SPMV_LONG
+                             ? __reduce_add_sync(FULL, n > 0 && n <= SPMV_LONG ? (int)n : 0) : 0;
+      const bool is_long = n > (sizeof(A) == 8 && filled < 32 * SPMV_SPARSE ? SPMV_SPARSE_LONG : SPMV_LONG);
       const int sn = is_long ? -1 : (int)n;  // a short row's entries
-      if (!ordered && __reduce_add_sync(FULL, sn < 0 ? 0 : sn) >= 32 * SPMV_MEAN4) {
+      if (!ordered && filled >= 32 * SPMV_MEAN4) {
         const int sub = lane & 3;
 #pragma unroll 1
         for (int b = lane >> 2; b < 32; b += 8) {
