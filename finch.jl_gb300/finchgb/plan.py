@@ -21,6 +21,10 @@ class Plan:
         self._A_desc = A.desc()
         desc.A = ctypes.addressof(self._A_desc)
         self._keep = keep  # the bound buffers stay alive with the plan
+        # the candidates are timed on a stream of the plan's own, which does not
+        # wait for operands still being made on the caller's
+        if torch.cuda.is_available() and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream().synchronize()
         h = ctypes.c_void_p()
         L.call("fgb_plan_create", dev.context(), ctypes.byref(desc), tune_reps, ctypes.byref(h))
         self.h = h
