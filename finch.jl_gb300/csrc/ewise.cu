@@ -127,13 +127,18 @@ __device__ __forceinline__ int ew_warp_below(const int* bi, int bbase, int nb, i
 // uniform rows of 16 + 16 69 -> 66.  Not staging where only coordinates are
 // read measured 83 there, 64 warps an SM against 48 66 against 75, and one
 // warp for the longest pairs 322 in place of 155.
-template <int MODE, class T, class PA, class PB>
+// One thread per fiber stays up to 10 % faster on uniform F64 rows of 5 to 16
+// entries a pair (23.6 us against 25.1 at 5), where its warps never wait for a
+// neighbour, and is 5 to 8 times slower on Zipf rows of the same mean; without
+// the blocks' barriers those took 84 us in place of 71.
+// STAGE: false for short fibers, see EW_STAGE_MEAN.
+template <int MODE, bool STAGE, class T, class PA, class PB>
 __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile_k(int64_t nf, int R, Fiber<PA> a, const T* __restrict__ va,
                                                         Fiber<PB> b, const T* __restrict__ vb, int op,
                                                         int64_t* __restrict__ cnt, const int64_t* __restrict__ optr,
                                                         int32_t* __restrict__ oidx, T* __restrict__ out) {
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ int s_idx[EW_CAP];
+  __shared__ int s_idx[STAGE ? EW_CAP : 1];
   __shared__ unsigned s_src[MODE == EW_FILL ? EW_CAP : 1];
   __shared__ int s_long[EW_THREADS];
   __shared__ int s_nlong;
@@ -142,9 +147,9 @@ __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t f0 = (int64_t)blockIdx.x * R;
   const int rows = nf - f0 < R ? (int)(nf - f0) : R;
-  const int64_t a0 = a.lo(f0), b0 = b.lo(f0);
-  const int64_t na = a.lo(f0 + rows) - a0, nb = b.lo(f0 + rows) - b0;
-  const bool staged = na + nb <= EW_CAP;
+  const int64_t a0 = STAGE ? a.lo(f0) : 0, b0 = STAGE ? b.lo(f0) : 0;
+  const int64_t na = STAGE ? a.lo(f0 + rows) - a0 : 0, nb = STAGE ? b.lo(f0 + rows) - b0 : 0;
+  const bool staged = STAGE && na + nb <= EW_CAP;
   if (tid == 0) s_nlong = 0;
   int64_t pa = 0, pb = 0;  // the thread's fiber, from the tile's first entries
   int64_t la = 0, lb = 0;
@@ -206,6 +211,23 @@ __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile
   if (tid < rows) {
     if (la + lb > EW_LONG) {
       s_long[atomicAdd(&s_nlong, 1)] = tid;
+    } else if constexpr (!STAGE) {
+      const int *ai = a.idx + pa, *bi = b.idx + pb;
+      const int ea = (int)la, eb = (int)lb, shift = a.base - b.base;
+      int i = 0, j = 0, n = 0;
+      T acc = T(0);
+      while (i < ea && j < eb) {
+        const int ca = __ldg(ai + i), cb = __ldg(bi + j) + shift;
+        if (ca == cb) {
+          if constexpr (MODE == EW_REDUCE) acc = fused(va[pa + i], vb[pb + j], acc);
+          if constexpr (MODE == EW_SCATTER) atomicAdd(out + (ca - a.base), wmul(va[pa + i], vb[pb + j]));
+          ++n;
+        }
+        i += ca <= cb;
+        j += cb <= ca;
+      }
+      if (MODE == EW_COUNT) cnt[f0 + tid] = op == FGB_EW_ADD ? la + lb - n : n;
+      if (MODE == EW_REDUCE) out[f0 + tid] = acc;
     } else if (staged) {
       merge(s_idx + pa, 0, s_idx + na + pb, 0);
     } else {
@@ -464,14 +486,29 @@ static int ew_rows(const fgb_ctx* ctx, const fgb_sparse* A, const fgb_sparse* B)
   return (int)std::max<int64_t>(r, 1);
 }
 
+// Below this many entries a pair of fibers on average, the modes that write no
+// list read the coordinates where they lie: the copy into shared memory costs
+// a chain of loads and a barrier, and short lists come out of L1.  Row sums of
+// A .* B, F64, 873,496 uniform rows, staged against not: 5 a pair 31.2 / 25.1
+// us, 8 37.0 / 35.2, 12 52.4 / 48.4, 16 63.9 / 65.2, 24 104 / 119; sums
+// over rows 35.4 / 29.2, 41.6 / 39.5, 59.4 / 56.7, 72.2 / 76.5; Zipf rows
+// 73.8 / 71.4 to 158 / 155 at 16.
+constexpr double EW_STAGE_MEAN = 14;
 template <int MODE, class T>
 static int ew_tile(fgb_ctx* ctx, const fgb_sparse* A, const fgb_sparse* B, int op, int64_t* cnt, const int64_t* optr,
                    int32_t* oidx, T* out, cudaStream_t s) {
   const int64_t nf = n_fibers(A);
   const int R = ew_rows(ctx, A, B);
+  const unsigned blocks = (unsigned)((nf + R - 1) / R);
   return with_fibers(A, B, [&](auto fa, auto fb) {
-    ew_tile_k<MODE><<<(unsigned)((nf + R - 1) / R), EW_THREADS, 0, s>>>(nf, R, fa, (const T*)A->val, fb,
-                                                                       (const T*)B->val, op, cnt, optr, oidx, out);
+    if constexpr (MODE != EW_FILL)
+      if ((double)A->nnz + (double)B->nnz < EW_STAGE_MEAN * (double)nf) {
+        ew_tile_k<MODE, false><<<blocks, EW_THREADS, 0, s>>>(nf, R, fa, (const T*)A->val, fb, (const T*)B->val, op,
+                                                             cnt, optr, oidx, out);
+        return check_launch("ew_tile_k");
+      }
+    ew_tile_k<MODE, true><<<blocks, EW_THREADS, 0, s>>>(nf, R, fa, (const T*)A->val, fb, (const T*)B->val, op, cnt,
+                                                        optr, oidx, out);
     return check_launch("ew_tile_k");
   });
 }

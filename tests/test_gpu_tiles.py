@@ -134,6 +134,9 @@ def ewise_pair(kind, rng, dtype):
     elif kind == "long":  # long pairs in staged tiles and beyond them
         la = rng.integers(0, 6, 500)
         la[[3, 4, 100, 499]] = (33, 64, 700, 9000)
+    elif kind == "rare":  # short fibers on average, read where they lie, and a few long pairs among them
+        la = rng.integers(0, 5, 5003)
+        la[[3, 4, 90, 700, 5002]] = (33, 64, 300, 9000, 700)
     elif kind == "one":
         la = np.array([5000])
     else:  # nothing, or nothing in one of the two
@@ -151,7 +154,7 @@ def ewise_pair(kind, rng, dtype):
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32, np.int32, np.int64])
-@pytest.mark.parametrize("kind", ["short", "long", "one", "none"])
+@pytest.mark.parametrize("kind", ["short", "long", "rare", "one", "none"])
 def test_ewise_tiles(gpu_lib, kind, dtype):
     """Merges of short pairs (a thread each, staged) and long ones (a warp
     each, staged or not), with ptr widths and index bases of their own:
