@@ -65,39 +65,52 @@ __global__ void __launch_bounds__(256) spmv_csr_pull(int64_t nrows, const PtrT* 
 // No sampled row longer than `cut`: `lanes` lanes per row, grid-strided, as
 // spmv_csr_pull.  The groups of a warp are never made to meet (a ballot per
 // row would have them wait for the longest of their rows: 171 against 140 us
-// on the 4M-node graph), so a row of more than 32 * lanes entries that the
-// sample missed goes to a list.
+// on the 4M-node graph), so a row of more than `limit` entries, which the
+// sample missed, goes to a list.  Groups of 8 keep four sums a lane where rows
+// average over 24 entries: a row's 32 sums, and its bits, are those of 32
+// lanes, at fewer FP64 instructions (FP64, 400,000 rows of 100: 195 us, by
+// equal shares with a warp a row 310).
 //
-// A longer row among them: the walk over rows and stored entries (row r sits
-// at step r + ptr[r]) is cut into equal shares, one a warp, and a warp owns
-// the rows that begin in its share: no row is split, no partial sums leave a
-// warp, and a warp that meets long rows has fewer others.  It searches ptr
-// for its first row and takes the rows 32 at a time: one of at most SPMV_LONG
-// entries by its own lane, or, where the 32 rows average SPMV_MEAN4 entries,
-// by 4 lanes (a lane's loads are uncoalesced: long enough rows pay for the
-// two shuffles); a longer row by the whole warp, one of more than SPMV_BLOCK
-// entries by way of the list.  Where the 32 rows average fewer than
-// SPMV_SPARSE entries of 8 bytes, rows over SPMV_SPARSE_LONG count as long:
-// the few lanes that had one kept the warp, and FP64 its pipe, busy for as
-// many steps (Zipf 1M x 16, FP64, 153 -> 139 us; 4M x 2 118 -> 103).  For
-// 4-byte values it gains 2-7 % there, but the 32-register build then spills
-// and the 4M-node graph loses 5 %.
+// A longer row among them, or rows long on average (`cut` -1): the walk over
+// rows and stored entries (row r sits at step r + ptr[r]) is cut into equal
+// shares, one a warp, and a warp owns the rows that begin in its share: no row
+// is split, no partial sums leave a warp, and a warp that meets long rows has
+// fewer others.  It searches ptr for its first row and takes the rows 32 at a
+// time: one of at most SPMV_LONG entries by its own lane, or, where the 32
+// rows average SPMV_MEAN4 entries, by 4 lanes (a lane's loads are uncoalesced: long
+// enough rows pay for the two shuffles); a longer row by the whole warp, one
+// of more than SPMV_BLOCK entries by way of the list.  Where the 32 rows
+// average fewer than SPMV_SPARSE entries of 8 bytes, rows over
+// SPMV_SPARSE_LONG count as long: the few lanes that had one kept the warp,
+// and FP64 its pipe, busy for as many steps (Zipf 1M x 16, FP64, 153 -> 139
+// us; 4M x 2 118 -> 103).  For 4-byte values it gains 2-7 % there, but the
+// 4-byte builds spill as it is (28 to 40 bytes at the 32 registers that keep
+// 64 warps an SM), more with the rule, and the 4M-node graph loses 5 %.
 //
 // When a block's warps are done they share its list, the longest rows by the
-// whole block; a full list is no loss but in speed.  `ordered`
-// (FGB_FINCH_ORDER) folds every row as one running value, j ascending: a long
-// row's entries are loaded 32 at a time and folded in order by every lane.
+// whole block.  Which rows the list takes, and so a row's order of summation,
+// depends on the matrix alone: lane groups that leave more than it holds have
+// it filled again, run by run, and a warp lists the first of its own rows.
+// `ordered` (FGB_FINCH_ORDER) folds every row as one running value, j
+// ascending: a long row's entries are loaded 32 at a time and folded in order
+// by every lane, in FP64 32 times a lane's own work for the pipe; so evenly
+// long rows stay with their lanes where there are rows enough to fill the
+// device (FP64, 400,000 rows of 50: 167 against 1,160 us by their warps).
 //
 // Bound: the gathers of x (one L1 tag a clock per SM), FP64 folds also by the
-// FP64 pipe.  GB300, per call, against rows of at most 32 entries on a lane
-// and longer ones by their warp in turn, with the contraction chosen at run
-// time: Zipf 1M x 16 FP64 283 -> 145 us with three operands in rotation; uniform 4M x 8: FP64 360 -> 183, FP32 156 -> 142, Int32 min-plus
-// 149 -> 140.  Staging tiles of entries in shared memory (coalesced, every
-// row folded from there) measured 298 (FP64) and 184 (FP32) on the uniform
+// FP64 pipe.  GB300, per call behind a cold L2, against fixed groups of 8 or
+// 32 lanes or, over 311,296 rows, one lane for rows up to 32 entries and a
+// warp for longer ones, with the contraction chosen at run time: Zipf 1M x 16
+// FP64 281 -> 136 us, FP32 165 -> 103; uniform 4M x 8 FP64 365 -> 184, FP32
+// 166 -> 144, Int32 min-plus 166 -> 144; rows of 4,000, 2,000 of them, FP64
+// 82 -> 53, FP32 73 -> 46; 64 rows of 100,000, FP32, 1,205 -> 124.  The sample
+// costs a uniform matrix about 1 us: 20,000 rows of 16, FP32, 3.2 -> 4.3 us in
+// a graph.  Staging tiles of entries in shared memory (coalesced, every row
+// folded from there) measured 298 (FP64) and 184 (FP32) on the uniform 4M
 // rows, and equal shares alone 194 and 162.
 constexpr int SPMV_LONG = 32, SPMV_SPARSE_LONG = 16, SPMV_SPARSE = 6;
 constexpr int SPMV_BLOCK = 2048;  // a warp alone takes 8 us for one
-constexpr int SPMV_LIST = 64;  // rows a block can leave to the end
+constexpr int SPMV_LIST = 64;  // rows a block can leave to the end (a longer list costs L1)
 constexpr int SPMV_MEAN4 = 14;
 
 // First row whose step ptr[r] - f0 + r is at least `target` (nrows if none),
@@ -129,9 +142,10 @@ __global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int
                                                         const int* __restrict__ idx,
                                                         const VT* __restrict__ val,
                                                         const A* __restrict__ x, A* __restrict__ y,
-                                                        int base, int accumulate, int ordered, int lanes,
-                                                        int64_t cut) {
+                                                        int base, int accumulate, int ordered, int lanes, int sums,
+                                                        int64_t cut, int limit) {
   using S = Semi<SR, A>;
+  using IT = typename std::conditional<sizeof(PtrT) == 4, uint32_t, int64_t>::type;  // an entry's position
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int WARPS = 8;
   __shared__ A s_red[WARPS];
@@ -140,6 +154,9 @@ __global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t warp = (int64_t)blockIdx.x * WARPS + w;
   const int64_t nwarps = (int64_t)gridDim.x * WARPS;
+  // the thread's first row by lane groups, read beside the sample
+  const int64_t first = (blockIdx.x * 256u + threadIdx.x) / (unsigned)lanes;
+  IT p0 = 0, p1 = 0;
   bool over = false;
 #pragma unroll
   for (int u = 0; u < 32 / WARPS; ++u) {
@@ -149,11 +166,39 @@ __global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int
   if (threadIdx.x == 0) s_n = 0;
   const bool skewed = __syncthreads_or(over);
 
-  auto fold_long = [&](int64_t row, int64_t q0, int64_t q1) {  // one row by the warp
+  constexpr std::integral_constant<bool, sizeof(A) == 8> wide{};
+  auto term = [&](A acc, IT p) { return S::step(acc, to_acc<A>(val[p]), __ldg(x + (__ldg(idx + p) - base)), FM); };
+  // Entries p, p + stride, ... below p1, added to `acc` in that order, four
+  // of them loaded at once.  AHEAD: their values before the gathers of x, not
+  // behind them (a choice of registers in flight, by measurement).
+  auto fold = [&](A acc, IT p, IT p1, int stride, auto ahead) -> A {
+    constexpr bool AHEAD = decltype(ahead)::value;
+    for (; p + 3 * stride < p1; p += 4 * stride) {
+      A a[4], xv[4];
+      int j[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        j[u] = __ldg(idx + p + u * stride);
+        if (AHEAD) a[u] = to_acc<A>(val[p + u * stride]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) xv[u] = __ldg(x + (j[u] - base));
+      if (!AHEAD)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] = to_acc<A>(val[p + u * stride]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc = S::step(acc, a[u], xv[u], FM);
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (p + u * stride < p1) acc = term(acc, p + u * stride);
+    return acc;
+  };
+  auto fold_long = [&](int64_t row, IT q0, IT q1) {  // one row by the warp
     A acc;
     if (ordered) {
       acc = accumulate ? y[row] : S::identity();
-      for (int64_t q = q0; q < q1; q += 32) {
+      for (IT q = q0; q < q1; q += 32) {
         A a = A(0), xv = A(0);
         if (q + lane < q1) {
           a = to_acc<A>(val[q + lane]);
@@ -165,12 +210,7 @@ __global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int
           acc = S::step(acc, __shfl_sync(FULL, a, u), __shfl_sync(FULL, xv, u), FM);
       }
     } else {
-      acc = S::identity();
-#pragma unroll 4
-      for (int64_t q = q0 + lane; q < q1; q += 32) {
-        const int j = __ldg(idx + q) - base;
-        acc = S::step(acc, to_acc<A>(val[q]), __ldg(x + j), FM);
-      }
+      acc = fold(S::identity(), q0 + lane, q1, 32, wide);
 #pragma unroll
       for (int m = 16; m >= 1; m >>= 1) acc = S::add(acc, shfl_xor(FULL, acc, m, 32));
       if (accumulate) acc = S::add(y[row], acc);
@@ -178,73 +218,85 @@ __global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int
     if (lane == 0) y[row] = acc;
   };
 
-  // Leaves a row to the end; false if the list is full.
-  auto leave = [&](int64_t row) -> bool {
-    const int at = atomicAdd(&s_n, 1);
-    if (at < SPMV_LIST) s_row[at] = row;
-    return at < SPMV_LIST;
-  };
-
-  auto by_lanes = [&](auto lanes_c) {
-    constexpr int G = decltype(lanes_c)::value;
+  // G lanes a row, U running sums a lane: entry p of a row is added to the
+  // row's sum p mod G * U, and the sums are folded as a tree.
+  auto by_lanes = [&](auto lanes_c, auto sums_c) {
+    constexpr int G = decltype(lanes_c)::value, U = decltype(sums_c)::value;
     const int sub = lane % G;
     const int64_t ngroups = nwarps * 32 / G;
-    for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G; row < nrows; row += ngroups) {
-      const int64_t p0 = ld_ptr(ptr, row) - base, p1 = ld_ptr(ptr, row + 1) - base;
-      if (p1 - p0 > 32 * G) {  // not sampled: the warps of the block fold it afterwards
-        int kept = 0;
-        if (sub == 0) kept = leave(row) ? 1 : 0;
-        if (__shfl_sync(group_mask<G>(), kept, 0, G)) continue;
+    for (int64_t row = first; row < nrows; row += ngroups) {
+      p0 = (IT)(ld_ptr(ptr, row) - base);
+      p1 = (IT)(ld_ptr(ptr, row + 1) - base);
+      if (p1 - p0 > (IT)limit) {  // not sampled: the warps of the block fold it afterwards
+        if (sub == 0) {
+          const int at = atomicAdd(&s_n, 1);
+          if (at < SPMV_LIST) s_row[at] = row;
+        }
+        continue;
       }
-      A acc = G == 1 && accumulate ? y[row] : S::identity();
-#pragma unroll 4
-      for (int64_t p = p0 + sub; p < p1; p += G) {
-        const int j = __ldg(idx + p) - base;
-        acc = S::step(acc, to_acc<A>(val[p]), __ldg(x + j), FM);
+      A acc[U];
+      acc[0] = G == 1 && accumulate ? y[row] : S::identity();
+#pragma unroll
+      for (int u = 1; u < U; ++u) acc[u] = S::identity();
+      if constexpr (U == 1) {
+        acc[0] = fold(acc[0], p0 + sub, p1, G, std::true_type{});
+      } else {
+        for (IT p = p0 + sub; p < p1; p += G * U) {
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (p + u * G < p1) acc[u] = term(acc[u], p + u * G);
+        }
+#pragma unroll
+        for (int h = U / 2; h >= 1; h >>= 1)
+#pragma unroll
+          for (int u = 0; u < h; ++u) acc[u] = S::add(acc[u], acc[u + h]);
       }
       if (G > 1) {
 #pragma unroll
-        for (int m = G / 2; m >= 1; m >>= 1) acc = S::add(acc, shfl_xor(group_mask<G>(), acc, m, G));
-        if (sub == 0) y[row] = accumulate ? S::add(y[row], acc) : acc;
+        for (int m = G / 2; m >= 1; m >>= 1) acc[0] = S::add(acc[0], shfl_xor(group_mask<G>(), acc[0], m, G));
+        if (sub == 0) y[row] = accumulate ? S::add(y[row], acc[0]) : acc[0];
       } else {
-        y[row] = acc;
+        y[row] = acc[0];
       }
     }
   };
   if (!skewed) {
-    if (lanes == 1) by_lanes(std::integral_constant<int, 1>{});
-    else if (lanes == 4) by_lanes(std::integral_constant<int, 4>{});
-    else by_lanes(std::integral_constant<int, 8>{});
+    using std::integral_constant;
+    if (lanes == 1) by_lanes(integral_constant<int, 1>{}, integral_constant<int, 1>{});
+    else if (lanes == 4) by_lanes(integral_constant<int, 4>{}, integral_constant<int, 1>{});
+    else if (lanes == 32) by_lanes(integral_constant<int, 32>{}, integral_constant<int, 1>{});
+    else if (sums == 1) by_lanes(integral_constant<int, 8>{}, integral_constant<int, 1>{});
+    else by_lanes(integral_constant<int, 8>{}, integral_constant<int, 4>{});
   } else {
     const int64_t f0 = ld_ptr(ptr, 0);
     const int64_t entries = ld_ptr(ptr, nrows) - f0;
     const int64_t per = (entries + nrows + nwarps - 1) / nwarps;
     const int64_t end = (warp + 1) * per;
     int64_t r0 = spmv_step_row(nrows, ptr, f0, entries, warp * per, lane);
+    int listed = 0;
     while (true) {  // warp-uniform
       const int64_t row = r0 + lane;
-      int64_t p0 = 0, n = -1;  // -1: not this warp's row
+      p0 = p1 = 0;
+      bool mine = false;
       if (row < nrows) {
-        p0 = ld_ptr(ptr, row) - base;
-        n = ld_ptr(ptr, row + 1) - base - p0;
-        if (p0 + base - f0 + row >= end) n = -1;
+        const int64_t at = ld_ptr(ptr, row), to = ld_ptr(ptr, row + 1);
+        mine = at - f0 + row < end;
+        p0 = (IT)(at - base);
+        p1 = mine ? (IT)(to - base) : p0;
       }
+      const IT n = p1 - p0;
       const int filled = sizeof(A) == 8 || !ordered  // entries in rows of at most SPMV_LONG
-                             ? __reduce_add_sync(FULL, n > 0 && n <= SPMV_LONG ? (int)n : 0) : 0;
-      const bool is_long = n > (sizeof(A) == 8 && filled < 32 * SPMV_SPARSE ? SPMV_SPARSE_LONG : SPMV_LONG);
-      const int sn = is_long ? -1 : (int)n;  // a short row's entries
+                             ? __reduce_add_sync(FULL, n <= SPMV_LONG ? (int)n : 0) : 0;
+      const bool is_long = n > (IT)(ordered ? limit : sizeof(A) == 8 && filled < 32 * SPMV_SPARSE ? SPMV_SPARSE_LONG : SPMV_LONG);
+      const int sn = is_long || !mine ? -1 : (int)n;  // a short row's entries
       if (!ordered && filled >= 32 * SPMV_MEAN4) {
         const int sub = lane & 3;
 #pragma unroll 1
         for (int b = lane >> 2; b < 32; b += 8) {
-          const int64_t q0 = __shfl_sync(FULL, p0, b);
+          const IT q0 = __shfl_sync(FULL, p0, b);
           const int bn = __shfl_sync(FULL, sn, b);
           A acc = S::identity();
-#pragma unroll 4
-          for (int k = sub; k < bn; k += 4) {
-            const int j = __ldg(idx + q0 + k) - base;
-            acc = S::step(acc, to_acc<A>(val[q0 + k]), __ldg(x + j), FM);
-          }
+          if (bn > 0) acc = fold(acc, q0 + sub, q0 + bn, 4, wide);
           acc = S::add(acc, shfl_xor(FULL, acc, 2, 32));
           acc = S::add(acc, shfl_xor(FULL, acc, 1, 32));
           if (sub == 0 && bn >= 0) y[r0 + b] = accumulate ? S::add(y[r0 + b], acc) : acc;
@@ -254,57 +306,71 @@ __global__ void __launch_bounds__(256, sizeof(A) == 8 ? 6 : 8) spmv_csr_auto(int
         const int* ix = idx + p0;
         const VT* vx = val + p0;
 #pragma unroll 4
-        for (int k = 0; k < sn; ++k) {
-          const int j = __ldg(ix + k) - base;
-          acc = S::step(acc, to_acc<A>(vx[k]), __ldg(x + j), FM);
-        }
+        for (int k = 0; k < sn; ++k) acc = S::step(acc, to_acc<A>(vx[k]), __ldg(x + (__ldg(ix + k) - base)), FM);
         y[row] = acc;
       }
       unsigned longs = __ballot_sync(FULL, is_long);
       while (longs) {
         const int l = __ffs(longs) - 1;
         longs &= longs - 1;
-        const int64_t q0 = __shfl_sync(FULL, p0, l), m = __shfl_sync(FULL, n, l);
-        if (m > SPMV_BLOCK && !ordered) {
-          int kept = 0;
-          if (lane == 0) kept = leave(r0 + l) ? 1 : 0;
-          if (__shfl_sync(FULL, kept, 0)) continue;
+        const IT q0 = __shfl_sync(FULL, p0, l), m = __shfl_sync(FULL, n, l);
+        if (m > SPMV_BLOCK && !ordered && listed < SPMV_LIST / WARPS) {  // never more than the list holds
+          if (lane == 0) s_row[atomicAdd(&s_n, 1)] = r0 + l;
+          ++listed;
+          continue;
         }
         fold_long(r0 + l, q0, q0 + m);
       }
-      if (__shfl_sync(FULL, (int)(n < 0), 31)) break;  // the warp's rows end here
+      if (!__shfl_sync(FULL, (int)mine, 31)) break;  // the warp's rows end here
       r0 += 32;
     }
   }
 
   __syncthreads();
-  const int left = s_n < SPMV_LIST ? s_n : SPMV_LIST;
-  for (int l = w; l < left; l += WARPS) {
-    const int64_t row = s_row[l];
-    const int64_t q0 = ld_ptr(ptr, row) - base, q1 = ld_ptr(ptr, row + 1) - base;
-    if (ordered || q1 - q0 <= SPMV_BLOCK) fold_long(row, q0, q1);
-  }
-  if (ordered) return;
-  for (int l = 0; l < left; ++l) {  // block-uniform: the longest by the whole block
-    const int64_t row = s_row[l];
-    const int64_t q0 = ld_ptr(ptr, row) - base, q1 = ld_ptr(ptr, row + 1) - base;
-    if (q1 - q0 <= SPMV_BLOCK) continue;
-    A acc = S::identity();
-#pragma unroll 4
-    for (int64_t q = q0 + threadIdx.x; q < q1; q += 32 * WARPS) {
-      const int j = __ldg(idx + q) - base;
-      acc = S::step(acc, to_acc<A>(val[q]), __ldg(x + j), FM);
+  // Lane groups may leave more than the list holds: it is then filled again
+  // from SPMV_LIST of the block's rows at a time, so which rows the warps fold
+  // does not depend on who came first.
+  const bool again = s_n > SPMV_LIST;
+  const int round = 256 / lanes;  // rows the block's groups take at once
+  int64_t rb = (int64_t)blockIdx.x * round, part = 0;
+  do {  // block-uniform
+    if (again) {
+      __syncthreads();
+      if (threadIdx.x == 0) s_n = 0;
+      __syncthreads();
+      const int64_t row = rb + part + threadIdx.x;
+      if (threadIdx.x < SPMV_LIST && part + threadIdx.x < round && row < nrows &&
+          ld_ptr(ptr, row + 1) - ld_ptr(ptr, row) > limit)
+        s_row[atomicAdd(&s_n, 1)] = row;
+      __syncthreads();
+      part += SPMV_LIST;
+      if (part >= round) {
+        part = 0;
+        rb += (int64_t)gridDim.x * round;
+      }
     }
+    const int left = s_n;
+    for (int l = w; l < left; l += WARPS) {
+      const int64_t row = s_row[l];
+      const IT q0 = (IT)(ld_ptr(ptr, row) - base), q1 = (IT)(ld_ptr(ptr, row + 1) - base);
+      if (ordered || q1 - q0 <= SPMV_BLOCK) fold_long(row, q0, q1);
+    }
+    for (int l = 0; l < left && !ordered; ++l) {  // block-uniform: the longest by the whole block
+      const int64_t row = s_row[l];
+      const IT q0 = (IT)(ld_ptr(ptr, row) - base), q1 = (IT)(ld_ptr(ptr, row + 1) - base);
+      if (q1 - q0 <= SPMV_BLOCK) continue;
+      A acc = fold(S::identity(), q0 + threadIdx.x, q1, 32 * WARPS, wide);
 #pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) acc = S::add(acc, shfl_xor(FULL, acc, m, 32));
-    if (lane == 0) s_red[w] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int v = 1; v < WARPS; ++v) acc = S::add(acc, s_red[v]);
-      y[row] = accumulate ? S::add(y[row], acc) : acc;
+      for (int m = 16; m >= 1; m >>= 1) acc = S::add(acc, shfl_xor(FULL, acc, m, 32));
+      if (lane == 0) s_red[w] = acc;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int v = 1; v < WARPS; ++v) acc = S::add(acc, s_red[v]);
+        y[row] = accumulate ? S::add(y[row], acc) : acc;
+      }
+      __syncthreads();
     }
-    __syncthreads();
-  }
+  } while (again && rb < nrows);
 }
 
 template <int SR, class VT, class A, class PtrT, int G, bool PATTERN>
@@ -442,11 +508,35 @@ static int launch_typed(fgb_ctx* ctx, const fgb_sparse* A_, const void* x, void*
         // fill the device, one, and 4 from 14 entries a row (8-byte values:
         // 1M x 8 rows 52 against 64 us, x 24 rows 176 against 131) or from 6
         // (4-byte: 4M x 2 rows 41 against 74, x 8 rows 148 against 142); with
-        // fewer rows more lanes, so that more of the device works.
+        // fewer rows more lanes, so that more of the device works.  Over 24
+        // entries a row (32 with many rows) 8 lanes with four sums each; 32
+        // lanes where 8 a row leave 4-byte rows over 64 entries short of
+        // warps (8,192 x 400, FP32: 14.4 us, by 8 27).  Equal shares, a warp
+        // a row, from 160 entries a row (FP64 8,192 x 400 25 us, by 8 lanes
+        // 51; 8,192 x 100 16.6 against 12.8; FP32 400,000 x 200 314 against
+        // 329, x 100 187 against 176), few 4-byte rows from 640 (70,000 x 200
+        // 67 against 44 by 8 lanes, 2,000 x 4,000 46 against 73).
         const bool many = nf >= (int64_t)ctx->num_sms * 2048;
-        const int lanes = ordered ? 1 : many ? (avg < (sizeof(A) == 8 ? SPMV_MEAN4 : 6) ? 1 : 4)
-                                             : avg <= 2.0 ? 1 : avg <= 8.0 || sizeof(A) == 8 ? 4 : 8;
-        const int64_t cut = std::max<int64_t>(SPMV_LONG, (int64_t)(4.0 * avg));
+        const bool wide = sizeof(A) == 8;
+        int lanes = avg <= 2.0 ? 1 : avg <= 8.0 || wide ? 4 : 8, sums = 1;
+        bool shares = false;
+        if (ordered) lanes = 1;
+        else if (avg > (many ? 32 : 24)) {
+          shares = avg > (wide || many ? 160 : 640);
+          lanes = avg > 64 && nf * 8 < (int64_t)ctx->num_sms * 2048 && !wide ? 32 : 8;
+          sums = lanes == 32 ? 1 : 4;
+        } else if (many) lanes = avg < (wide ? SPMV_MEAN4 : 6) ? 1 : 4;
+        const int64_t spread = std::max<int64_t>(SPMV_LONG, (int64_t)(4.0 * avg));
+        // A row that the sample would accept is not one that it missed.  In
+        // Finch's order long rows go to their warps where they are fewer than
+        // about the resident warps, which is where a lane's chain is longer
+        // (FP64: 1,000 x 1,000 103 us by warps, 462 by lanes; 70,000 x 50 214
+        // against 37; FP32, whose pipe is wider, 8,192 x 400 44 against 111).
+        int64_t cut = spread, limit = std::max<int64_t>(32 * lanes, avg > 24 ? spread : 0);
+        if (ordered) limit = avg > 24 && nf > (int64_t)ctx->num_sms * (wide ? 48 : 160) ? spread : SPMV_LONG;
+        if (avg > 24 || !ordered) cut = std::min(cut, limit);
+        limit = std::min<int64_t>(limit, 1 << 30);
+        if (shares) cut = -1;
         auto go = [&](auto fmc) {
           auto kern = spmv_csr_auto<SR, VT, A, PtrT, decltype(fmc)::value>;
           static const int occ = [&] {  // once per process (one device model); thread-safe
@@ -457,7 +547,7 @@ static int launch_typed(fgb_ctx* ctx, const fgb_sparse* A_, const void* x, void*
           const int64_t need = (steps + 8 * 64 - 1) / (8 * 64);  // at least 64 steps a warp
           const int grid = (int)std::min<int64_t>(need, (int64_t)occ * ctx->num_sms);
           kern<<<grid, threads, 0, s>>>(nf, ptr, idx, val, (const A*)x, (A*)y, base, accumulate, ordered ? 1 : 0,
-                                        lanes, cut);
+                                        lanes, sums, cut, (int)limit);
         };
         bool unfused = false;
         if constexpr (SR == SR_PT && std::is_floating_point<A>::value) {

@@ -1,0 +1,65 @@
+"""Matrices whose rows are long, all of them or where a sample of the rows does
+not show it: every row is summed in an order that its length alone decides."""
+import numpy as np
+import pytest
+
+from finchgb import _lib as L
+from finchgb import device as dev
+from helpers import assert_close, abs_terms, oracle_spmv, to_dev, to_host, upload
+from test_gpu_tiles import csr_of_lengths
+
+pytestmark = pytest.mark.gpu
+
+
+def strided_sums(b, x, rows, parts=32):
+    """The rows' sums as `parts` running sums, entry p of a row in sum
+    p mod parts, folded as a tree; products and sums each rounded."""
+    out = []
+    for r in rows:
+        p0, p1 = b.ptr[r] - 1, b.ptr[r + 1] - 1
+        t = b.val[p0:p1] * x[b.idx[p0:p1] - 1]
+        t = np.concatenate([t, np.zeros(-t.size % parts, t.dtype)]).reshape(-1, parts)
+        acc = np.zeros(parts, t.dtype)
+        for row in t:
+            acc = acc + row
+        while acc.size > 1:
+            acc = acc[:acc.size // 2] + acc[acc.size // 2:]
+        out.append(acc[0])
+    return np.array(out)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("m,length", [(3000, 28), (3000, 63), (3000, 100), (600, 129), (500, 161), (300, 400), (40, 2048),
+                                      (50_000, 40)])
+def test_spmv_evenly_long_rows(gpu_lib, m, length, dtype):
+    """Rows of one length over 24: 32 sums a row, whichever lanes hold them,
+    and one running sum in Finch's order."""
+    rng = np.random.default_rng(length)
+    b = csr_of_lengths(rng, np.full(m, length), 5000, dtype)
+    A, x = upload(b), rng.standard_normal(5000).astype(dtype)
+    rows = np.unique(np.concatenate([[0, m - 1], rng.integers(0, m, 60)]))
+    got = to_host(dev.spmv(A, to_dev(x), flags=L.NO_FMA))
+    assert np.array_equal(got[rows], strided_sums(b, x, rows))
+    assert_close(got, oracle_spmv(L.PLUS_TIMES, b, x), abs_terms(b, x), dtype)
+    got = to_host(dev.spmv(A, to_dev(x), flags=L.FINCH_ORDER))
+    assert np.array_equal(got, oracle_spmv(L.PLUS_TIMES, b, x, fma=True))
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("m,short,length", [(320_000, 2, 40), (90_000, 6, 300), (60_000, 20, 300)])
+def test_spmv_unsampled_long_rows(gpu_lib, m, short, length, dtype):
+    """More long rows together, between the sampled ones, than a block's list
+    holds: each is summed as if it were alone, so twice the same."""
+    rng = np.random.default_rng(short)
+    lengths = np.full(m, short)
+    long = np.arange(m // 64, m // 64 + 700)  # half a sampling step from the windows
+    lengths[long] = length
+    b = csr_of_lengths(rng, lengths, 9000, dtype)
+    A, x = upload(b), rng.standard_normal(9000).astype(dtype)
+    got = to_host(dev.spmv(A, to_dev(x), flags=L.NO_FMA))
+    rows = rng.choice(long, 200, replace=False)
+    assert np.array_equal(got[rows], strided_sums(b, x, rows))
+    assert_close(got, oracle_spmv(L.PLUS_TIMES, b, x), abs_terms(b, x), dtype)
+    assert np.array_equal(got, to_host(dev.spmv(A, to_dev(x), flags=L.NO_FMA)))
+    got = to_host(dev.spmv(A, to_dev(x), flags=L.FINCH_ORDER))
+    assert np.array_equal(got, oracle_spmv(L.PLUS_TIMES, b, x, fma=True))
