@@ -63,3 +63,18 @@ def test_spmv_unsampled_long_rows(gpu_lib, m, short, length, dtype):
     assert np.array_equal(got, to_host(dev.spmv(A, to_dev(x), flags=L.NO_FMA)))
     got = to_host(dev.spmv(A, to_dev(x), flags=L.FINCH_ORDER))
     assert np.array_equal(got, oracle_spmv(L.PLUS_TIMES, b, x, fma=True))
+
+
+@pytest.mark.parametrize("mean", [3, 12])
+def test_spmv_short_rows_of_skewed_fp32(gpu_lib, mean):
+    """Rows of at most 32 entries beside long ones: FP32 keeps four sums a row,
+    also where the rows around it are nearly empty."""
+    rng = np.random.default_rng(mean)
+    lengths = np.where(rng.random(60_000) < 0.2, rng.integers(5, 33, 60_000), mean // 3)
+    lengths[::500] = 900
+    b = csr_of_lengths(rng, lengths, 9000, np.float32)
+    A, x = upload(b), rng.standard_normal(9000).astype(np.float32)
+    got = to_host(dev.spmv(A, to_dev(x), flags=L.NO_FMA))
+    rows = rng.choice(np.flatnonzero((lengths > 4) & (lengths <= 32)), 300, replace=False)
+    assert np.array_equal(got[rows], strided_sums(b, x, rows, parts=4))
+    assert_close(got, oracle_spmv(L.PLUS_TIMES, b, x), abs_terms(b, x), np.float32)
