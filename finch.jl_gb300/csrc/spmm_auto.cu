@@ -1,42 +1,88 @@
-// CSR SpMM of aligned operands with no schedule given: whole rows, blocks of
-// equal work.
+// CSR SpMM of aligned operands with no schedule given: blocks of equal work.
 //
 // Row r sits at step r + ptr[r] of the walk over rows and stored entries, and
 // a block owns the rows that begin in its share of the steps; it searches ptr
-// for the first of them.  A group of G lanes (V columns a lane) folds one row
-// at a time, one running sum per output, with up to 8 gathers of B in flight;
-// the groups of a warp are never made to meet.  A row of more than SA_LONG
-// entries is listed, and when the block's other rows are done the whole block
-// folds each listed row, an equal part per group, the parts added in a fixed
-// order.  No row is split between blocks: no scratch, no second launch, and
-// results are the same run to run.
+// for the first of them.  A group of G lanes (V columns a lane) folds a row of
+// at most SA_ROW entries, with up to 8 gathers of B in flight; the groups of a
+// warp are never made to meet.  Longer rows are listed, and when the block's
+// others are done the whole block folds them one after another, an equal part
+// per group, the parts added in a fixed order.
 //
-// Bound: latency of the B-row gathers (8 a lane in flight, 2 blocks of 126
-// registers an SM: 3 or 4 blocks spill and measured 137 and 116 us where 2
-// take 102), FP64 also by its pipe.  GB300, per call, against the merge-path
-// items it replaces as the default (the warp's sub-groups met at every row
-// end, and carries were fixed up afterwards): 150,011 rows, 120,007 columns,
-// 12 entries a row, k = 64: F32 Zipf 194 -> 102 us, uniform 152 -> 90; F64
-// Zipf 414 -> 295, uniform 406 -> 262.  20,000 Zipf rows 102 -> 31; 100,000
-// rows of 20, k = 128, 234 -> 139; 500,000 rows of 8, k = 32, 279 -> 174.
+// No row is split between blocks: no scratch, no second launch, and results are
+// the same run to run.
+//
+// A lane keeps 4 sums a column in FP32 (8 for up to 16 columns; FP64, whose
+// pipe waits for the adds, 32 / G, at most 4): at least as many as sub-groups
+// of a warp shared a row in the merge path, so that FP32 rounds no more.
+//
+// Bound: latency of the B-row gathers (8 a lane in flight, 3 blocks of 80
+// registers an SM; with 2 blocks of 96 a fifth slower), FP64 also by its pipe.
+// GB300, per call behind a cold L2, against the merge-path items that were the
+// default before (the warp's sub-groups met at every row end, and carries were
+// fixed up afterwards): 150,000 rows of 12, 120,000 columns, k = 64: F32 Zipf
+// 204 -> 103 us, uniform 157 -> 69; F64 396 -> 286, 412 -> 245.  20,000 Zipf
+// rows 98 -> 40; 100,000 rows of 30, k = 128, 252 -> 140.
 #include <algorithm>
+#include <type_traits>
 
 #include "spmm_common.cuh"
 
 namespace fgb {
 
 constexpr int SA_THREADS = 256;
-constexpr int SA_LONG = 64;
-constexpr int SA_LIST = 64;  // more than a share holds; a full list would cost speed only
+constexpr int SA_ROW = 64;
+constexpr int SA_LIST = 64;  // a share of SA_MAX_STEPS holds the beginnings of at most 32 rows over SA_ROW entries
 // A block's share: an equal one of all steps while that keeps every block in
-// the first wave, at most SA_MAX_STEPS (4096: 500,000 rows of 8 189 us).
+// the first wave, at most SA_MAX_STEPS (with 4096, 150,000 rows of 12, k = 64,
+// 79 us in place of 66, 300,000 rows of 4 97 for 80).
 constexpr int64_t SA_MIN_STEPS = 256, SA_MAX_STEPS = 2048;
+// Running sums a lane keeps for each column.
+template <class T, int G>
+__host__ __device__ constexpr int sa_sums() {
+  return sizeof(T) == 4 ? (G == 4 ? 8 : 4) : G == 4 ? 4 : 32 / G;
+}
+
+// The sum that a batch's u-th entry goes to.  Eight entries are spread evenly
+// over the sums.  What is left of a row goes in pairs, three in one: a row of
+// up to 4 has its products fused into its sums, which rounds less there than
+// sums of one product each (4 entries, FP32: relative error 3.6e-8 for 3.8e-8;
+// 24 entries: 3.9e-8 by 4 or 8 sums, 7.4e-8 by one).
+template <int N>
+using Int = std::integral_constant<int, N>;
+enum SaBatch { SA_EIGHT, SA_LOW4, SA_HIGH4, SA_FOUR, SA_REST };
+template <SaBatch K>
+using Kind = std::integral_constant<SaBatch, K>;
+template <int U, SaBatch K>
+__device__ constexpr int sa_sum(int u) {
+  return K == SA_EIGHT ? u * U / 8 : K == SA_LOW4 ? u : K == SA_HIGH4 ? 4 + u : (K == SA_FOUR ? u / 2 : 2) % U;
+}
+
+// NB entries of a row from the t-th of the group's current ones; lane l of the
+// group holds entries l, l + G, ...
+template <class T, int G, int V, int U, int E, int NB, SaBatch K>
+__device__ __forceinline__ void sa_batch(VecT<T, V> (&acc)[U], int t, const int (&my_j)[E], const T (&my_a)[E],
+                                         const T* __restrict__ Bc, int64_t ldb, unsigned gmask, uint64_t pol) {
+  VecT<T, V> b[NB];
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    const int j = __shfl_sync(gmask, E == 1 || t + u < G ? my_j[0] : my_j[E - 1], t + u, G);
+    b[u] = gather<T, V>(Bc + (int64_t)j * ldb, pol);
+  }
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    const T a = __shfl_sync(gmask, E == 1 || t + u < G ? my_a[0] : my_a[E - 1], t + u, G);
+    acc_step<T, V>(acc[sa_sum<U, K>(u)], a, b[u], FM_FMA);
+  }
+}
 
 template <class T, class VT, class PtrT, int G, int V>
-__global__ void __launch_bounds__(SA_THREADS, 2) spmm_csr_auto(
+__global__ void __launch_bounds__(SA_THREADS, 3) spmm_csr_auto(
     int64_t nrows, const PtrT* __restrict__ ptr, const int* __restrict__ idx, const VT* __restrict__ val,
     const T* __restrict__ B, int64_t ldb, T* __restrict__ C, int64_t ldc, int64_t c0, int64_t nk, int base,
     int accumulate) {
+  using IT = typename std::conditional<sizeof(PtrT) == 4, uint32_t, int64_t>::type;  // an entry's position
+  constexpr int E = G < 8 ? 8 / G : 1;
+  constexpr int U = sa_sums<T, G>();
   constexpr int NG = SA_THREADS / G, WARPS = SA_THREADS / 32;
   __shared__ int64_t s_long[SA_LIST];
   __shared__ int s_n;
@@ -45,7 +91,7 @@ __global__ void __launch_bounds__(SA_THREADS, 2) spmm_csr_auto(
   const unsigned gmask = group_mask<G>();
   const int64_t col = c0 + (int64_t)lane * V;
   const bool active = col < nk;  // V divides nk - c0
-  const T* Bc = B + col;
+  const T* Bc = B + (active ? col : c0);  // lanes past nk gather what the group's first does, and store nothing
   const uint64_t pol_stream = policy_evict_first();
   const uint64_t pol_keep = policy_evict_last();
   const int64_t f0 = ld_ptr(ptr, 0);
@@ -69,31 +115,58 @@ __global__ void __launch_bounds__(SA_THREADS, 2) spmm_csr_auto(
   }
   __syncthreads();
 
-  // Entries [p, p1) of a row by the group, in storage order.
-  auto fold = [&](VecT<T, V>& acc, int64_t p, int64_t p1) {
-    for (int64_t pb = p; pb < p1; pb += G) {
-      const int64_t pe = pb + lane;
-      int my_j = 0;
-      T my_a = T(0);
-      if (pe < p1) {
-        my_j = ld_stream_i32(idx + pe, pol_stream) - base;
-        my_a = load_val<T, VT>(val, pe, pol_stream);
+  // The sum of entries [p, p1) of a row by the group.
+  auto fold = [&](IT p, IT p1) -> VecT<T, V> {
+    VecT<T, V> acc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < V; ++q) acc[u].v[q] = T(0);
+    for (IT pb = p; pb < p1; pb += G * E) {
+      int my_j[E];
+      T my_a[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const IT pe = pb + lane + e * G;
+        my_j[e] = 0;
+        my_a[e] = T(0);
+        if (pe < p1) {
+          my_j[e] = ld_stream_i32(idx + pe, pol_stream) - base;
+          my_a[e] = load_val<T, VT>(val, pe, pol_stream);
+        }
       }
-      const int cnt = p1 - pb < (int64_t)G ? (int)(p1 - pb) : G;
+      const int cnt = p1 - pb < (IT)(G * E) ? (int)(p1 - pb) : G * E;
+      auto batch = [&](auto nb, auto kind, int t) {
+        sa_batch<T, G, V, U, E, decltype(nb)::value, decltype(kind)::value>(acc, t, my_j, my_a, Bc, ldb, gmask,
+                                                                            pol_keep);
+      };
       int t = 0;
-      if constexpr (G >= 8)
-        for (; t + 8 <= cnt; t += 8)
-          pull_batch<T, G, V, 8, FM_FMA>(acc, t, my_j, my_a, Bc, ldb, active, gmask, pol_keep);
+      if constexpr (U == 8) {  // 4 gathers ahead: 8 sums of 4 columns take the registers
+        if (cnt == 8) {
+          batch(Int<4>{}, Kind<SA_LOW4>{}, 0);
+          batch(Int<4>{}, Kind<SA_HIGH4>{}, 4);
+          t = 8;
+        }
+      } else {
+        for (; t + 8 <= cnt; t += 8) batch(Int<8>{}, Kind<SA_EIGHT>{}, t);
+      }
       if (t + 4 <= cnt) {
-        pull_batch<T, G, V, 4, FM_FMA>(acc, t, my_j, my_a, Bc, ldb, active, gmask, pol_keep);
+        batch(Int<4>{}, Kind<SA_FOUR>{}, t);
         t += 4;
       }
       if (t + 2 <= cnt) {
-        pull_batch<T, G, V, 2, FM_FMA>(acc, t, my_j, my_a, Bc, ldb, active, gmask, pol_keep);
+        batch(Int<2>{}, Kind<SA_REST>{}, t);
         t += 2;
       }
-      if (t < cnt) pull_batch<T, G, V, 1, FM_FMA>(acc, t, my_j, my_a, Bc, ldb, active, gmask, pol_keep);
+      if (t < cnt) batch(Int<1>{}, Kind<SA_REST>{}, t);
     }
+#pragma unroll
+    for (int h = U / 2; h >= 1; h >>= 1)
+#pragma unroll
+      for (int u = 0; u < h; ++u)
+#pragma unroll
+        for (int q = 0; q < V; ++q) acc[u].v[q] += acc[u + h].v[q];
+    return acc[0];
   };
   auto store = [&](int64_t row, VecT<T, V> acc) {
     T* dst = C + row * ldc + col;
@@ -104,49 +177,49 @@ __global__ void __launch_bounds__(SA_THREADS, 2) spmm_csr_auto(
     }
     store_out<T, V>(dst, acc, pol_stream);
   };
-
   for (int64_t row = lo + g; row < nrows; row += NG) {
     const int64_t p0 = ld_ptr(ptr, row), p1 = ld_ptr(ptr, row + 1);
     if (p0 - f0 + row >= end) break;
-    if (p1 - p0 > SA_LONG) {
+    if (p1 - p0 > SA_ROW) {
       int kept = 0;
       if (lane == 0) {
         const int at = atomicAdd(&s_n, 1);
         if (at < SA_LIST) s_long[at] = row;
-        kept = at < SA_LIST;
+        kept = at < SA_LIST;  // always, if ptr ends where the host was told
       }
       if (__shfl_sync(gmask, kept, 0, G)) continue;
     }
-    VecT<T, V> acc;
-#pragma unroll
-    for (int q = 0; q < V; ++q) acc.v[q] = T(0);
-    fold(acc, p0 - base, p1 - base);
+    const VecT<T, V> acc = fold((IT)(p0 - base), (IT)(p1 - base));
     if (active) store(row, acc);
   }
   __syncthreads();
   const int nlong = s_n < SA_LIST ? s_n : SA_LIST;
+  int turn = 0;
   for (int l = 0; l < nlong; ++l) {  // block-uniform
-    const int64_t row = s_long[l];
-    const int64_t p0 = ld_ptr(ptr, row) - base, p1 = ld_ptr(ptr, row + 1) - base;
-    const int64_t part = ((p1 - p0 + NG - 1) / NG + 7) / 8 * 8;
+    const int64_t row = s_long[l], p0 = ld_ptr(ptr, row), p1 = ld_ptr(ptr, row + 1);
+    const int quantum = sizeof(T) == 4 ? 8 : 16;
+    const int64_t part = ((p1 - p0 + NG - 1) / NG + quantum - 1) / quantum * quantum;
     const int64_t q0 = p0 + g * part, q1 = q0 + part < p1 ? q0 + part : p1;
     VecT<T, V> acc;
 #pragma unroll
     for (int q = 0; q < V; ++q) acc.v[q] = T(0);
-    fold(acc, q0, q1);
-    __syncwarp();
+    if (__any_sync(0xffffffffu, q0 < p1)) {  // warps with nothing to add leave the FP64 pipe to the others
+      acc = fold((IT)(q0 < p1 ? q0 - base : 0), (IT)(q0 < p1 ? q1 - base : 0));
+      __syncwarp();
 #pragma unroll
-    for (int m = G; m < 32; m <<= 1)
+      for (int m = G; m < 32; m <<= 1)
 #pragma unroll
-      for (int q = 0; q < V; ++q) acc.v[q] += __shfl_xor_sync(0xffffffffu, acc.v[q], m);
-    if ((tid & 31) < G) s_part[l & 1][tid >> 5][lane] = acc;
+        for (int q = 0; q < V; ++q) acc.v[q] += __shfl_xor_sync(0xffffffffu, acc.v[q], m);
+    }
+    turn ^= 1;  // the other half of s_part: one barrier a row
+    if ((tid & 31) < G) s_part[turn][tid >> 5][lane] = acc;
     __syncthreads();
-    if (tid < G && active) {
+    if (tid < G) {
 #pragma unroll
       for (int w = 1; w < WARPS; ++w)
 #pragma unroll
-        for (int q = 0; q < V; ++q) acc.v[q] += s_part[l & 1][w][lane].v[q];
-      store(row, acc);
+        for (int q = 0; q < V; ++q) acc.v[q] += s_part[turn][w][lane].v[q];
+      if (active) store(row, acc);
     }
   }
 }
@@ -177,13 +250,16 @@ template <class T, class VT>
 static int auto_typed(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk, void* C, int64_t ldc,
                       int accumulate, cudaStream_t s) {
   constexpr int V = sizeof(T) == 4 ? 4 : 2;
-  const int64_t need = (nk + V - 1) / V;  // lanes that cover a row of B, at most a warp
+  const int64_t lanes = (nk + V - 1) / V;  // that cover a row of B, at most a warp
   auto go = [&](auto ptr_t) -> int {
     using P = decltype(ptr_t);
-    if (need <= 4) return launch_auto<T, VT, P, 4>(ctx, A, (const T*)B, ldb, nk, (T*)C, ldc, accumulate, s);
-    if (need <= 8) return launch_auto<T, VT, P, 8>(ctx, A, (const T*)B, ldb, nk, (T*)C, ldc, accumulate, s);
-    if (need <= 16) return launch_auto<T, VT, P, 16>(ctx, A, (const T*)B, ldb, nk, (T*)C, ldc, accumulate, s);
-    return launch_auto<T, VT, P, 32>(ctx, A, (const T*)B, ldb, nk, (T*)C, ldc, accumulate, s);
+    auto run = [&](auto g) {
+      return launch_auto<T, VT, P, decltype(g)::value>(ctx, A, (const T*)B, ldb, nk, (T*)C, ldc, accumulate, s);
+    };
+    if (lanes <= 4) return run(Int<4>{});
+    if (lanes <= 8) return run(Int<8>{});
+    if (lanes <= 16) return run(Int<16>{});
+    return run(Int<32>{});
   };
   return A->ptr_t == FGB_I32 ? go(int32_t(0)) : go(int64_t(0));
 }

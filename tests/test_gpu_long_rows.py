@@ -5,7 +5,7 @@ import pytest
 
 from finchgb import _lib as L
 from finchgb import device as dev
-from helpers import assert_close, abs_terms, oracle_spmv, to_dev, to_host, upload
+from helpers import abs_terms, assert_close, oracle_spmv, to_dev, to_host, upload
 from test_gpu_tiles import csr_of_lengths
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +78,23 @@ def test_spmv_short_rows_of_skewed_fp32(gpu_lib, mean):
     rows = rng.choice(np.flatnonzero((lengths > 4) & (lengths <= 32)), 300, replace=False)
     assert np.array_equal(got[rows], strided_sums(b, x, rows, parts=4))
     assert_close(got, oracle_spmv(L.PLUS_TIMES, b, x), abs_terms(b, x), np.float32)
+
+
+def swallowing(lengths, n, dtype):
+    """Rows whose first product swallows every later one that is added to it,
+    one by one: 2^24 (FP64: 2^53), then ones.  What a row's sum lacks is how
+    many entries shared a running sum with the first."""
+    b = csr_of_lengths(np.random.default_rng(1), lengths, n, dtype)
+    b.val[:] = 1
+    b.val[(b.ptr[:-1] - 1)[np.asarray(lengths) > 0]] = 2.0 ** (24 if dtype == np.float32 else 53)
+    return b, np.ones(n, dtype)
+
+
+@pytest.mark.parametrize("nk", [4, 16, 20, 48, 64, 128])
+def test_spmm_fp32_rows_have_four_sums(gpu_lib, nk):
+    """The default for aligned operands, rows of at most 64 entries: no more
+    than a quarter of a row shares its first entry's sum."""
+    lengths = np.repeat([64, 48, 32, 16], 100)
+    b, _ = swallowing(lengths, 300, np.float32)
+    C = to_host(dev.spmm(upload(b), to_dev(np.ones((300, nk), np.float32))))
+    assert (C.astype(np.float64) >= 2.0 ** 24 + (lengths - lengths / 4)[:, None]).all()
