@@ -4,9 +4,11 @@
 // a block owns the rows that begin in its share of the steps; it searches ptr
 // for the first of them.  A group of G lanes (V columns a lane) folds a row of
 // at most SA_ROW entries, with up to 8 gathers of B in flight; the groups of a
-// warp are never made to meet.  Longer rows are listed, and when the block's
-// others are done the whole block folds them one after another, an equal part
-// per group, the parts added in a fixed order.
+// warp are never made to meet.  Longer rows are listed and taken when the
+// block's others are done: where there are a few of them, one a warp, an equal
+// part per group of it (rows up to SA_WARP entries); else, and longer ones, by
+// the whole block one after another, an equal part per group of the block, the
+// parts added in a fixed order.
 //
 // No row is split between blocks: no scratch, no second launch, and results are
 // the same run to run.
@@ -21,7 +23,10 @@
 // default before (the warp's sub-groups met at every row end, and carries were
 // fixed up afterwards): 150,000 rows of 12, 120,000 columns, k = 64: F32 Zipf
 // 204 -> 103 us, uniform 157 -> 69; F64 396 -> 286, 412 -> 245.  20,000 Zipf
-// rows 98 -> 40; 100,000 rows of 30, k = 128, 252 -> 140.
+// rows 98 -> 40; 100,000 rows of 30, k = 128, 252 -> 140.  Rows of 100 (50,000),
+// k = 16 / 64 / 128, F32 96 -> 106, 236 -> 158, 344 -> 224; of 400 (20,000) 114
+// -> 125, 325 -> 214, 488 -> 306 (one row after another by the block, at 2
+// blocks an SM, 336 / 284 / 364 and 151 / 272 / 356).
 #include <algorithm>
 #include <type_traits>
 
@@ -36,6 +41,10 @@ constexpr int SA_LIST = 64;  // a share of SA_MAX_STEPS holds the beginnings of 
 // the first wave, at most SA_MAX_STEPS (with 4096, 150,000 rows of 12, k = 64,
 // 79 us in place of 66, 300,000 rows of 4 97 for 80).
 constexpr int64_t SA_MIN_STEPS = 256, SA_MAX_STEPS = 2048;
+// Rows up to this length may be a warp's: 128 entries a group of it, at most
+// 512; none in FP64 where a warp is one group with one sum a lane.
+template <class T, int G>
+constexpr int SA_WARP = G <= 8 ? 512 : sizeof(T) == 8 && G == 32 ? 0 : 4096 / G;
 // Running sums a lane keeps for each column.
 template <class T, int G>
 __host__ __device__ constexpr int sa_sums() {
@@ -81,7 +90,7 @@ __global__ void __launch_bounds__(SA_THREADS, 3) spmm_csr_auto(
     const T* __restrict__ B, int64_t ldb, T* __restrict__ C, int64_t ldc, int64_t c0, int64_t nk, int base,
     int accumulate) {
   using IT = typename std::conditional<sizeof(PtrT) == 4, uint32_t, int64_t>::type;  // an entry's position
-  constexpr int E = G < 8 ? 8 / G : 1;
+  constexpr int P = 32 / G, E = G < 8 ? 8 / G : 1;
   constexpr int U = sa_sums<T, G>();
   constexpr int NG = SA_THREADS / G, WARPS = SA_THREADS / 32;
   __shared__ int64_t s_long[SA_LIST];
@@ -194,32 +203,44 @@ __global__ void __launch_bounds__(SA_THREADS, 3) spmm_csr_auto(
   }
   __syncthreads();
   const int nlong = s_n < SA_LIST ? s_n : SA_LIST;
+  // Rows up to this length by the warps: from 4 of them that is sooner than a
+  // barrier a row.
+  const int by_warp = nlong >= 4 ? SA_WARP<T, G> : 0;
   int turn = 0;
-  for (int l = 0; l < nlong; ++l) {  // block-uniform
-    const int64_t row = s_long[l], p0 = ld_ptr(ptr, row), p1 = ld_ptr(ptr, row + 1);
-    const int quantum = sizeof(T) == 4 ? 8 : 16;
-    const int64_t part = ((p1 - p0 + NG - 1) / NG + quantum - 1) / quantum * quantum;
-    const int64_t q0 = p0 + g * part, q1 = q0 + part < p1 ? q0 + part : p1;
-    VecT<T, V> acc;
+#pragma unroll 1
+  for (int block = by_warp ? 0 : 1; block < 2; ++block) {  // the warps' rows, then the block's
+    const int step = block ? 1 : WARPS;
+#pragma unroll 1
+    for (int l = block ? 0 : tid >> 5; l < nlong; l += step) {  // block- or warp-uniform
+      const int64_t row = s_long[l], p0 = ld_ptr(ptr, row), p1 = ld_ptr(ptr, row + 1);
+      if ((p1 - p0 <= by_warp) == (block != 0)) continue;
+      const int quantum = sizeof(T) == 4 ? 8 : block ? 16 : 1;
+      const int parts = block ? NG : P, mine = block ? g : g % P;  // P groups a warp
+      const int64_t part = ((p1 - p0 + parts - 1) / parts + quantum - 1) / quantum * quantum;
+      const int64_t q0 = p0 + mine * part, q1 = q0 + part < p1 ? q0 + part : p1;
+      VecT<T, V> acc;
 #pragma unroll
-    for (int q = 0; q < V; ++q) acc.v[q] = T(0);
-    if (__any_sync(0xffffffffu, q0 < p1)) {  // warps with nothing to add leave the FP64 pipe to the others
-      acc = fold((IT)(q0 < p1 ? q0 - base : 0), (IT)(q0 < p1 ? q1 - base : 0));
-      __syncwarp();
+      for (int q = 0; q < V; ++q) acc.v[q] = T(0);
+      if (__any_sync(0xffffffffu, q0 < p1)) {  // warps with nothing to add leave the FP64 pipe to the others
+        acc = fold((IT)(q0 < p1 ? q0 - base : 0), (IT)(q0 < p1 ? q1 - base : 0));
+        __syncwarp();
 #pragma unroll
-      for (int m = G; m < 32; m <<= 1)
+        for (int m = G; m < 32; m <<= 1)
 #pragma unroll
-        for (int q = 0; q < V; ++q) acc.v[q] += __shfl_xor_sync(0xffffffffu, acc.v[q], m);
-    }
-    turn ^= 1;  // the other half of s_part: one barrier a row
-    if ((tid & 31) < G) s_part[turn][tid >> 5][lane] = acc;
-    __syncthreads();
-    if (tid < G) {
+          for (int q = 0; q < V; ++q) acc.v[q] += __shfl_xor_sync(0xffffffffu, acc.v[q], m);
+      }
+      if (block) {
+        turn ^= 1;  // the other half of s_part: one barrier a row
+        if ((tid & 31) < G) s_part[turn][tid >> 5][lane] = acc;
+        __syncthreads();
+        if (tid < G) {
 #pragma unroll
-      for (int w = 1; w < WARPS; ++w)
+          for (int w = 1; w < WARPS; ++w)
 #pragma unroll
-        for (int q = 0; q < V; ++q) acc.v[q] += s_part[turn][w][lane].v[q];
-      if (active) store(row, acc);
+            for (int q = 0; q < V; ++q) acc.v[q] += s_part[turn][w][lane].v[q];
+        }
+      }
+      if ((block ? tid < G : (tid & 31) < G) && active) store(row, acc);
     }
   }
 }

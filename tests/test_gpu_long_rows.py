@@ -3,9 +3,10 @@ not show it: every row is summed in an order that its length alone decides."""
 import numpy as np
 import pytest
 
+import oracle
 from finchgb import _lib as L
 from finchgb import device as dev
-from helpers import abs_terms, assert_close, oracle_spmv, to_dev, to_host, upload
+from helpers import abs_terms, assert_close, bf16_bits, oracle_spmv, to_dev, to_host, upload
 from test_gpu_tiles import csr_of_lengths
 
 pytestmark = pytest.mark.gpu
@@ -98,3 +99,21 @@ def test_spmm_fp32_rows_have_four_sums(gpu_lib, nk):
     b, _ = swallowing(lengths, 300, np.float32)
     C = to_host(dev.spmm(upload(b), to_dev(np.ones((300, nk), np.float32))))
     assert (C.astype(np.float64) >= 2.0 ** 24 + (lengths - lengths / 4)[:, None]).all()
+
+
+@pytest.mark.parametrize("dtype,bf16", [(np.float32, False), (np.float64, False), (np.float32, True)])
+@pytest.mark.parametrize("nk", [16, 32, 64, 128])
+@pytest.mark.parametrize("length", [64, 65, 127, 129, 257, 512, 513, 1500])
+def test_spmm_evenly_long_rows(gpu_lib, length, nk, dtype, bf16):
+    """Rows of one length: by the groups, by the warps, by the block, cut."""
+    rng = np.random.default_rng(length)
+    m = 40_000 // length
+    r = csr_of_lengths(rng, np.full(m, length), 6000, dtype)
+    B = rng.standard_normal((6000, nk)).astype(dtype)
+    A, Bd = upload(r, as_bf16=bf16), to_dev(B)
+    val = bf16_bits(r.val) if bf16 else r.val
+    want = oracle.spmm_csr(m, 6000, r.ptr, r.idx, val, B, bf16=bf16)
+    scale = oracle.spmm_csr(m, 6000, r.ptr, r.idx, np.abs(r.val).astype(np.float64), np.abs(B).astype(np.float64))
+    C = to_host(dev.spmm(A, Bd))
+    assert_close(C, want, scale, dtype)
+    assert np.array_equal(C, to_host(dev.spmm(A, Bd)))
