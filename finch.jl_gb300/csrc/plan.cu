@@ -172,9 +172,9 @@ int issue(fgb_plan* p, const Choice& c, cudaStream_t s, bool plan_ready) {
         return spmm_merge(p->ctx, &p->A, d.in0, d.ld_in0, d.k, d.out, d.ld_out, d.dtype,
                           (d.flags & FGB_ACCUMULATE) ? 1 : 0, c.lanes, c.path, p->scratch,
                           p->scratch_bytes, s, plan_ready, nullptr, c.variant);
-      if (spmm_aligned(p))  // no item length: whole rows, equal shares per block
+      if (spmm_aligned(p))  // no item length: equal shares per block
         return spmm_auto(p->ctx, &p->A, d.in0, d.ld_in0, d.k, d.out, d.ld_out, d.dtype,
-                         (d.flags & FGB_ACCUMULATE) ? 1 : 0, s);
+                         (d.flags & FGB_ACCUMULATE) ? 1 : 0, p->scratch, p->scratch_bytes, s);
       return spmm_impl(p->ctx, &p->A, d.in0, d.ld_in0, d.k, d.out, d.ld_out, d.dtype, d.flags,
                        c.lanes, 0, s);
     case FGB_PLAN_SDDMM:
@@ -213,7 +213,7 @@ std::vector<Choice> candidates(const fgb_plan* p) {
     }
     for (int l : {8, 16, 32})
       for (int64_t path : {128, 256, 512, 1024}) out.push_back(Choice{l, path, 1, 0});
-    // spmm_auto: whole rows, equal shares per block; the lanes are those it takes
+    // spmm_auto: equal shares per block; the lanes are those it takes
     const int64_t need = d.k / (d.dtype == FGB_F64 ? 2 : 4);
     out.push_back(Choice{need <= 4 ? 4 : need <= 8 ? 8 : need <= 16 ? 16 : 32, 0, 1, 0});
     if (d.dtype == FGB_F32)  // B rows staged by TMA into a shared-memory ring
@@ -288,6 +288,8 @@ int fgb_plan_create(fgb_ctx* ctx, const fgb_plan_desc* desc, int32_t tune_reps, 
       if (c.path > 0 && c.variant < 2)  // the merge-path schedules
         p->scratch_bytes = std::max(p->scratch_bytes,
                                     spmm_merge_scratch_bytes(p->A.nrows, p->A.nnz, p->d.k, esz, c.path));
+    if (spmm_aligned(p))
+      p->scratch_bytes = std::max(p->scratch_bytes, spmm_auto_scratch_bytes(ctx, &p->A, p->d.k, p->d.dtype));
     if (p->scratch_bytes) {
       e = cudaMalloc(&p->scratch, p->scratch_bytes);
       if (e != cudaSuccess) {

@@ -207,7 +207,8 @@ static int run_typed(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t l
                         ((uintptr_t)C % (VN * sizeof(T)) == 0);
     if (!(flags & FGB_FINCH_ORDER) && vec_ok) {
       if (variant == 0 && lanes <= 0 && path <= 0)
-        return spmm_auto(ctx, A, B, ldb, nk, C, ldc, sizeof(T) == 8 ? FGB_F64 : FGB_F32, accumulate, s);
+        return spmm_auto(ctx, A, B, ldb, nk, C, ldc, sizeof(T) == 8 ? FGB_F64 : FGB_F32, accumulate,
+                         nullptr, 0, s);
       default_merge_tuning(A, nk, sizeof(T), &lanes, &path);
       return spmm_merge(ctx, A, B, ldb, nk, C, ldc, sizeof(T) == 8 ? FGB_F64 : FGB_F32,
                         accumulate, lanes, path, nullptr, 0, s, false, nullptr, variant);

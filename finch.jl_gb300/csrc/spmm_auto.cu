@@ -10,8 +10,10 @@
 // the whole block one after another, an equal part per group of the block, the
 // parts added in a fixed order.
 //
-// No row is split between blocks: no scratch, no second launch, and results are
-// the same run to run.
+// A row of more entries than two shares hold steps is cut at the shares: the
+// block in whose share it begins writes its part to C, the others leave theirs
+// as carries, and spmm_auto_fixup adds a row's carries in the order of the
+// blocks.  Results are the same run to run.
 //
 // A lane keeps 4 sums a column in FP32 (8 for up to 16 columns; FP64, whose
 // pipe waits for the adds, 32 / G, at most 4): at least as many as sub-groups
@@ -26,7 +28,9 @@
 // rows 98 -> 40; 100,000 rows of 30, k = 128, 252 -> 140.  Rows of 100 (50,000),
 // k = 16 / 64 / 128, F32 96 -> 106, 236 -> 158, 344 -> 224; of 400 (20,000) 114
 // -> 125, 325 -> 214, 488 -> 306 (one row after another by the block, at 2
-// blocks an SM, 336 / 284 / 364 and 151 / 272 / 356).
+// blocks an SM, 336 / 284 / 364 and 151 / 272 / 356).  One row of a million
+// entries beside 200,000 of 8: k = 16 F32 1,294 -> 93, k = 64 F64 2,661 -> 351
+// (whole, in one block, 21,126).
 #include <algorithm>
 #include <type_traits>
 
@@ -88,7 +92,7 @@ template <class T, class VT, class PtrT, int G, int V>
 __global__ void __launch_bounds__(SA_THREADS, 3) spmm_csr_auto(
     int64_t nrows, const PtrT* __restrict__ ptr, const int* __restrict__ idx, const VT* __restrict__ val,
     const T* __restrict__ B, int64_t ldb, T* __restrict__ C, int64_t ldc, int64_t c0, int64_t nk, int base,
-    int accumulate) {
+    int accumulate, int64_t* __restrict__ carry_row, T* __restrict__ carry) {
   using IT = typename std::conditional<sizeof(PtrT) == 4, uint32_t, int64_t>::type;  // an entry's position
   constexpr int P = 32 / G, E = G < 8 ? 8 / G : 1;
   constexpr int U = sa_sums<T, G>();
@@ -107,6 +111,8 @@ __global__ void __launch_bounds__(SA_THREADS, 3) spmm_csr_auto(
   const int64_t steps = ld_ptr(ptr, nrows) - f0 + nrows;
   const int64_t per = (steps + gridDim.x - 1) / gridDim.x;
   const int64_t first = blockIdx.x * per, end = first + per;
+  const int64_t whole = carry ? 2 * per : INT64_MAX;  // longer rows are cut at the shares
+  pdl_allow_next();  // spmm_auto_fixup may be set up beside this launch
   if (tid == 0) s_n = 0;
   // first row whose step is at least `first` (nrows if none): 256 probes a round
   int64_t lo = 0, hi = nrows;
@@ -206,14 +212,33 @@ __global__ void __launch_bounds__(SA_THREADS, 3) spmm_csr_auto(
   // Rows up to this length by the warps: from 4 of them that is sooner than a
   // barrier a row.
   const int by_warp = nlong >= 4 ? SA_WARP<T, G> : 0;
+  // The part of a row that began in another share.
+  const int64_t cut = lo > 0 ? lo - 1 : 0;
+  int64_t c_first = 0, c_end = 0;
+  if (carry && lo > 0) {
+    const int64_t p0 = ld_ptr(ptr, cut) - f0, p1 = ld_ptr(ptr, cut + 1) - f0;
+    if (p1 - p0 > whole) {
+      c_first = first - cut;
+      c_end = p1 < end - cut ? p1 : end - cut;
+    }
+  }
+  const bool head = c_first < c_end;
+  if (carry && c0 == 0 && tid == 0) carry_row[blockIdx.x] = head ? cut : -1;
   int turn = 0;
 #pragma unroll 1
   for (int block = by_warp ? 0 : 1; block < 2; ++block) {  // the warps' rows, then the block's
     const int step = block ? 1 : WARPS;
 #pragma unroll 1
-    for (int l = block ? 0 : tid >> 5; l < nlong; l += step) {  // block- or warp-uniform
-      const int64_t row = s_long[l], p0 = ld_ptr(ptr, row), p1 = ld_ptr(ptr, row + 1);
-      if ((p1 - p0 <= by_warp) == (block != 0)) continue;
+    for (int l = block ? (head ? -1 : 0) : tid >> 5; l < nlong; l += step) {  // block- or warp-uniform
+      int64_t row = cut, p0 = c_first + f0, p1 = c_end + f0;
+      if (l >= 0) {
+        row = s_long[l];
+        p0 = ld_ptr(ptr, row);
+        p1 = ld_ptr(ptr, row + 1);
+        const bool cutting = p1 - p0 > whole;
+        if ((p1 - p0 <= by_warp && !cutting) == (block != 0)) continue;
+        if (cutting && p1 > f0 + end - row) p1 = f0 + end - row;  // the rest is the next blocks'
+      }
       const int quantum = sizeof(T) == 4 ? 8 : block ? 16 : 1;
       const int parts = block ? NG : P, mine = block ? g : g % P;  // P groups a warp
       const int64_t part = ((p1 - p0 + parts - 1) / parts + quantum - 1) / quantum * quantum;
@@ -240,14 +265,61 @@ __global__ void __launch_bounds__(SA_THREADS, 3) spmm_csr_auto(
             for (int q = 0; q < V; ++q) acc.v[q] += s_part[turn][w][lane].v[q];
         }
       }
-      if ((block ? tid < G : (tid & 31) < G) && active) store(row, acc);
+      if (block ? tid >= G : (tid & 31) >= G) continue;
+      if (!active) continue;
+      if (l >= 0) {
+        store(row, acc);
+      } else {
+#pragma unroll
+        for (int q = 0; q < V; ++q) carry[blockIdx.x * nk + col + q] = acc.v[q];
+      }
     }
   }
 }
 
+// Adds the carries of every row that was cut to it: a block per row, its
+// carries in S consecutive runs, the runs in order.
+template <class T, class PtrT>
+__global__ void __launch_bounds__(SA_THREADS) spmm_auto_fixup(int64_t nrows, const PtrT* __restrict__ ptr,
+                                                             int64_t nblocks, int64_t nk,
+                                                             const int64_t* __restrict__ carry_row,
+                                                             const T* __restrict__ carry, T* __restrict__ C,
+                                                             int64_t ldc) {
+  __shared__ T s_sum[SA_THREADS];
+  pdl_wait_prev();
+  const int64_t f0 = ld_ptr(ptr, 0);
+  const int64_t per = (ld_ptr(ptr, nrows) - f0 + nrows + nblocks - 1) / nblocks;
+  int width = 4;  // columns at a time, a power of two
+  while (width < nk && width < SA_THREADS) width *= 2;
+  const int runs = SA_THREADS / width, run = threadIdx.x / width;
+  for (int64_t w = blockIdx.x; w < nblocks; w += gridDim.x) {  // block-uniform
+    const int64_t r = carry_row[w];
+    if (r < 0 || (w > 0 && carry_row[w - 1] == r)) continue;
+    const int64_t n = (ld_ptr(ptr, r + 1) - f0 - 1 + r) / per - w + 1;  // its carries, up to its last entry's block
+    const int64_t len = (n + runs - 1) / runs;
+    const int64_t a = w + run * len, b = a + len < w + n ? a + len : w + n;
+    for (int64_t c0 = 0; c0 < nk; c0 += width) {
+      const int64_t c = c0 + threadIdx.x % width;
+      T sum = T(0);
+      if (c < nk) {
+#pragma unroll 8
+        for (int64_t k = a; k < b; ++k) sum += carry[k * nk + c];
+      }
+      s_sum[threadIdx.x] = sum;
+      __syncthreads();
+      if (run == 0 && c < nk) {
+        for (int q = 1; q < runs; ++q) sum += s_sum[q * width + threadIdx.x];
+        C[r * ldc + c] += sum;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// `need` given: only the scratch that the call takes.
 template <class T, class VT, class PtrT, int G>
 static int launch_auto(fgb_ctx* ctx, const fgb_sparse* A, const T* B, int64_t ldb, int64_t nk, T* C, int64_t ldc,
-                       int accumulate, cudaStream_t s) {
+                       int accumulate, char* scratch, size_t* need, cudaStream_t s) {
   constexpr int V = sizeof(T) == 4 ? 4 : 2;
   auto kern = spmm_csr_auto<T, VT, PtrT, G, V>;
   static const int occ = [&] {  // once per process (one device model); thread-safe
@@ -258,24 +330,45 @@ static int launch_auto(fgb_ctx* ctx, const fgb_sparse* A, const T* B, int64_t ld
   const int64_t steps = A->nrows + A->nnz;
   const int64_t share = std::clamp(steps / ((int64_t)occ * ctx->num_sms), SA_MIN_STEPS, SA_MAX_STEPS);
   const int grid = (int)std::min<int64_t>((steps + share - 1) / share, INT32_MAX);
+  // no row is cut where the matrix is no wider than that
+  const size_t rows_bytes = (sizeof(int64_t) * grid + 255) & ~size_t(255);
+  if (need) {
+    *need = grid > 1 && A->ncols > 2 * share ? rows_bytes + sizeof(T) * grid * nk : 0;
+    return FGB_OK;
+  }
+  int64_t* carry_row = (int64_t*)scratch;
+  T* carry = scratch ? (T*)(scratch + rows_bytes) : nullptr;
   for (int64_t c0 = 0; c0 < nk; c0 += G * V) {
     kern<<<grid, SA_THREADS, 0, s>>>(A->nrows, (const PtrT*)A->ptr, (const int*)A->idx, (const VT*)A->val, B, ldb, C,
-                                     ldc, c0, nk, A->index_base, accumulate);
+                                     ldc, c0, nk, A->index_base, accumulate, carry_row, carry);
     const int rc = check_launch("spmm_csr_auto");
     if (rc) return rc;
   }
-  return FGB_OK;
+  if (!carry) return FGB_OK;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min<int64_t>(grid, 8 * ctx->num_sms));
+  cfg.blockDim = dim3(SA_THREADS);
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, spmm_auto_fixup<T, PtrT>, A->nrows, (const PtrT*)A->ptr, (int64_t)grid, nk,
+                     (const int64_t*)carry_row, (const T*)carry, C, ldc);
+  return check_launch("spmm_auto_fixup");
 }
 
 template <class T, class VT>
 static int auto_typed(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk, void* C, int64_t ldc,
-                      int accumulate, cudaStream_t s) {
+                      int accumulate, char* scratch, size_t* need, cudaStream_t s) {
   constexpr int V = sizeof(T) == 4 ? 4 : 2;
   const int64_t lanes = (nk + V - 1) / V;  // that cover a row of B, at most a warp
   auto go = [&](auto ptr_t) -> int {
     using P = decltype(ptr_t);
     auto run = [&](auto g) {
-      return launch_auto<T, VT, P, decltype(g)::value>(ctx, A, (const T*)B, ldb, nk, (T*)C, ldc, accumulate, s);
+      return launch_auto<T, VT, P, decltype(g)::value>(ctx, A, (const T*)B, ldb, nk, (T*)C, ldc, accumulate, scratch,
+                                                       need, s);
     };
     if (lanes <= 4) return run(Int<4>{});
     if (lanes <= 8) return run(Int<8>{});
@@ -285,12 +378,32 @@ static int auto_typed(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t 
   return A->ptr_t == FGB_I32 ? go(int32_t(0)) : go(int64_t(0));
 }
 
+static int auto_any(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk, void* C, int64_t ldc,
+                    int dtype, int accumulate, char* scratch, size_t* need, cudaStream_t s) {
+  if (dtype == FGB_F64)
+    return auto_typed<double, double>(ctx, A, B, ldb, nk, C, ldc, accumulate, scratch, need, s);
+  if (A->val_t == FGB_BF16)
+    return auto_typed<float, __nv_bfloat16>(ctx, A, B, ldb, nk, C, ldc, accumulate, scratch, need, s);
+  return auto_typed<float, float>(ctx, A, B, ldb, nk, C, ldc, accumulate, scratch, need, s);
+}
+
+size_t spmm_auto_scratch_bytes(fgb_ctx* ctx, const fgb_sparse* A, int64_t nk, int dtype) {
+  size_t need = 0;
+  if (A->nrows > 0 && nk > 0) auto_any(ctx, A, nullptr, 0, nk, nullptr, 0, dtype, 0, nullptr, &need, nullptr);
+  return need;
+}
+
 int spmm_auto(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk, void* C, int64_t ldc,
-              int dtype, int accumulate, cudaStream_t s) {
+              int dtype, int accumulate, void* scratch, size_t scratch_bytes, cudaStream_t s) {
   if (A->nrows == 0 || nk == 0) return FGB_OK;
-  if (dtype == FGB_F64) return auto_typed<double, double>(ctx, A, B, ldb, nk, C, ldc, accumulate, s);
-  if (A->val_t == FGB_BF16) return auto_typed<float, __nv_bfloat16>(ctx, A, B, ldb, nk, C, ldc, accumulate, s);
-  return auto_typed<float, float>(ctx, A, B, ldb, nk, C, ldc, accumulate, s);
+  const size_t need = spmm_auto_scratch_bytes(ctx, A, nk, dtype);
+  char* buf = need ? (char*)scratch : nullptr;
+  if (buf && scratch_bytes < need)
+    return set_error(FGB_EINVAL, "spmm: scratch of %zu bytes is below the %zu needed", scratch_bytes, need);
+  if (need && !buf) FGB_CUDA_TRY(cudaMallocAsync((void**)&buf, need, s));
+  const int rc = auto_any(ctx, A, B, ldb, nk, C, ldc, dtype, accumulate, buf, nullptr, s);
+  if (buf && !scratch) cudaFreeAsync(buf, s);
+  return rc;
 }
 
 }  // namespace fgb

@@ -73,10 +73,17 @@ int spmm_tma_items(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb
                    const int64_t* plan_k, int64_t* carry_row, void* carry, const int32_t* row_map,
                    int* err, cudaStream_t s);
 
-// Whole rows, equal shares of the rows and entries per block (spmm_auto.cu):
-// aligned CSR operands with no schedule given.
+// Equal shares of the rows and entries per block (spmm_auto.cu): aligned CSR
+// operands with no schedule given.  scratch == NULL allocates it on the stream.
+size_t spmm_auto_scratch_bytes(fgb_ctx* ctx, const fgb_sparse* A, int64_t nk, int dtype);
 int spmm_auto(fgb_ctx* ctx, const fgb_sparse* A, const void* B, int64_t ldb, int64_t nk, void* C, int64_t ldc,
-              int dtype, int accumulate, cudaStream_t s);
+              int dtype, int accumulate, void* scratch, size_t scratch_bytes, cudaStream_t s);
+
+// Programmatic dependent launch: lets the next launch of the stream start, and
+// waits for the previous one's end.  In a launch made without the attribute
+// both return at once.
+__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_prev() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class T, int V>
 struct VecT {

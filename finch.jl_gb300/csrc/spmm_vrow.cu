@@ -216,15 +216,12 @@ __global__ void vrow_gather_k(int64_t nv, const int32_t* __restrict__ ord,
     vr[i] = unsorted[ord[i]];
 }
 
-// Programmatic dependent launch: the launches of one SpMM after its first
-// may start while the previous one drains (its blocks take the SMs the
-// previous launch frees).  A launch signals at once that its successor may
-// start, waits for its predecessor before its first record that reads C
-// (w = -2, sorted last) and before it exits, so a launch that completes
-// implies that every earlier one did.  In a launch made without the
-// attribute both instructions return at once.
-__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait_prev() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Programmatic dependent launch (pdl_allow_next, pdl_wait_prev): the launches
+// of one SpMM after its first may start while the previous one drains (its
+// blocks take the SMs the previous launch frees).  A launch signals at once
+// that its successor may start, waits for its predecessor before its first
+// record that reads C (w = -2, sorted last) and before it exits, so a launch
+// that completes implies that every earlier one did.
 
 // The start of a virtual row: a light row's later column band (w = -2)
 // continues the running sum its earlier bands left in C, so the row is one

@@ -260,8 +260,9 @@ FGB_API int fgb_spmv(fgb_ctx* ctx, int semiring, const fgb_sparse* A, const void
  * (ldb), C row-major (ldc).  F32 (A F32 or BF16 values, B/C F32) or F64.
  * Replaces `@einsum C[i,k] += A[i,j]*B[j,k]` = tensordot(A,B,(2,1))
  * (src/interface/lazy.jl:215-257,387-404).  CSR runs load-balanced
- * (whole rows in equal shares of rows and entries per block, or column slabs
- * over virtual rows for a large B; deterministic); with FGB_FINCH_ORDER (or
+ * (equal shares of the rows and entries per block, rows longer than that cut
+ * and their parts added in order, or column slabs over virtual rows for a
+ * large B; deterministic); with FGB_FINCH_ORDER (or
  * an unaligned nk/ldb/ldc) each row is one running sum per column, j
  * ascending, bit-identical to Finch's nest.  CSC runs as a push with
  * atomics. */

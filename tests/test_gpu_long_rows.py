@@ -2,6 +2,7 @@
 not show it: every row is summed in an order that its length alone decides."""
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from finchgb import _lib as L
@@ -99,6 +100,45 @@ def test_spmm_fp32_rows_have_four_sums(gpu_lib, nk):
     b, _ = swallowing(lengths, 300, np.float32)
     C = to_host(dev.spmm(upload(b), to_dev(np.ones((300, nk), np.float32))))
     assert (C.astype(np.float64) >= 2.0 ** 24 + (lengths - lengths / 4)[:, None]).all()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("nk", [4, 32, 64, 128, 132])
+def test_spmm_hub_rows_are_cut(gpu_lib, nk, dtype):
+    """Rows of far more entries than a block's share of the steps: a share's
+    entries at most (2,048) share a sum with the first, and the parts of every
+    row meet in a fixed order; rows before, between and after them, a second
+    slab of columns, accumulating into strided rows."""
+    lengths = np.full(3000, 5)
+    lengths[[0, 700, 701, 2999]] = (60_000, 30_000, 21_000, 60_000)
+    n = 70_000
+    b, _ = swallowing(lengths, n, dtype)
+    big = 2.0 ** (24 if dtype == np.float32 else 53)
+    B = torch.ones((n, nk + 4), dtype=torch.float32 if dtype == np.float32 else torch.float64, device="cuda")[:, :nk]
+    for ptr in (lambda t: t, lambda t: t.long()):
+        A = upload(b)
+        A = dev.DeviceSparse(A.nrows, A.ncols, ptr(A.ptr), A.idx, A.val, A.orient, A.base)
+        C = torch.full((3000, nk + 4), 7.0, dtype=B.dtype, device="cuda")
+        dev.spmm(A, B, C[:, :nk])
+        got = to_host(C)[:, :nk].astype(np.float64) - big
+        lack = (lengths - 1)[:, None] - got
+        # adding the parts to the first rounds to even, once an addition: 3 + 3 + 7 + 1 of them at most
+        assert lack.min() >= -14 and lack.max() <= 2048 + 14
+        dev.spmm(A, B, C[:, :nk])
+        assert np.array_equal(to_host(C)[:, :nk].astype(np.float64) - big, got)
+        assert (to_host(C)[:, nk:] == 7).all()
+    A = upload(b)
+    A.val = torch.ones_like(A.val)
+    C = torch.full((3000, nk), 3.0, dtype=B.dtype, device="cuda")
+    dev.spmm(A, B, C, flags=L.ACCUMULATE)
+    assert np.array_equal(to_host(C), np.broadcast_to((lengths + 3.0)[:, None], (3000, nk)))
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s), torch.cuda.graph(g, stream=s):
+        dev.spmm(A, B, C)
+    C.zero_()
+    g.replay()
+    assert np.array_equal(to_host(C), np.broadcast_to(lengths[:, None], (3000, nk)))
 
 
 @pytest.mark.parametrize("dtype,bf16", [(np.float32, False), (np.float64, False), (np.float32, True)])
