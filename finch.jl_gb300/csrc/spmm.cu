@@ -28,8 +28,8 @@ namespace fgb {
 // bound by its pipe (one 32-lane FMA takes 16 clocks of an SM), where a
 // predicated-off update costs as much as a real one.  200,003 rows of 10, k =
 // 33, F64: 996 us with predicated batches of 8, the contraction chosen at run
-// time and 32 lanes for the 33rd column; 198 us now (the pipe's own time for
-// 66 M FMAs is 105).
+// time and 32 lanes for the 33rd column; 198 us then, 176 with no predicate for
+// lanes past the last column (the pipe's own time for 66 M FMAs is 105).
 template <class T, class VT, class PtrT, int G, int V, int FM>
 __global__ void __launch_bounds__(256, V == 1 ? 4 : 1) spmm_csr_pull(
     int64_t nrows, const PtrT* __restrict__ ptr, const int* __restrict__ idx,
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256, V == 1 ? 4 : 1) spmm_csr_pull(
   const int64_t ngroups = ((int64_t)gridDim.x * blockDim.x) / G;
   const int64_t col = c0 + (int64_t)lane * V;
   const bool active_col = col < nk;  // V divides nk - c0 in the vector path
-  const T* Bc = B + col;
+  const T* Bc = B + (active_col ? col : c0);
   const uint64_t pol_stream = policy_evict_first();
   const uint64_t pol_keep = policy_evict_last();
   for (int64_t row = group; row < nrows; row += ngroups) {
@@ -65,16 +65,16 @@ __global__ void __launch_bounds__(256, V == 1 ? 4 : 1) spmm_csr_pull(
       int t = 0;
       if constexpr (G >= 8)
         for (; t + 8 <= cnt; t += 8)
-          pull_batch<T, G, V, 8, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
+          pull_batch<T, G, V, 8, FM>(acc, t, my_j, my_a, Bc, ldb, gmask, pol_keep);
       if (t + 4 <= cnt) {
-        pull_batch<T, G, V, 4, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
+        pull_batch<T, G, V, 4, FM>(acc, t, my_j, my_a, Bc, ldb, gmask, pol_keep);
         t += 4;
       }
       if (t + 2 <= cnt) {
-        pull_batch<T, G, V, 2, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
+        pull_batch<T, G, V, 2, FM>(acc, t, my_j, my_a, Bc, ldb, gmask, pol_keep);
         t += 2;
       }
-      if (t < cnt) pull_batch<T, G, V, 1, FM>(acc, t, my_j, my_a, Bc, ldb, active_col, gmask, pol_keep);
+      if (t < cnt) pull_batch<T, G, V, 1, FM>(acc, t, my_j, my_a, Bc, ldb, gmask, pol_keep);
     }
     if (active_col) store_out<T, V>(C + row * ldc + col, acc, pol_stream);
   }

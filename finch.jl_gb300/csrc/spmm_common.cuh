@@ -152,14 +152,15 @@ __device__ __forceinline__ void acc_step(VecT<T, V>& acc, T a, const VecT<T, V>&
 
 // NB entries of a row, all of them stored: gathers first, then the updates in
 // storage order.  my_j/my_a: entry pb + lane of the group's current G entries.
+// Every lane gathers: one past the last column from a valid one.
 template <class T, int G, int V, int NB, int FM>
 __device__ __forceinline__ void pull_batch(VecT<T, V>& acc, int t, int my_j, T my_a, const T* __restrict__ Bc,
-                                           int64_t ldb, bool active, unsigned gmask, uint64_t pol) {
+                                           int64_t ldb, unsigned gmask, uint64_t pol) {
   VecT<T, V> b[NB];
 #pragma unroll
   for (int u = 0; u < NB; ++u) {
     const int j = __shfl_sync(gmask, my_j, t + u, G);
-    if (active) b[u] = gather<T, V>(Bc + (int64_t)j * ldb, pol);
+    b[u] = gather<T, V>(Bc + (int64_t)j * ldb, pol);
   }
 #pragma unroll
   for (int u = 0; u < NB; ++u) acc_step<T, V>(acc, __shfl_sync(gmask, my_a, t + u, G), b[u], FM);
