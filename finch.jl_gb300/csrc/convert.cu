@@ -8,6 +8,7 @@
 // histogram of c and an exclusive scan, like SparseList's freeze_level!
 // prefix sum (sparse_list_levels.jl:310-327).
 #include <cub/cub.cuh>
+#include <type_traits>
 
 #include "fiber_chunk.cuh"
 
@@ -19,15 +20,15 @@ namespace fgb {
 // fiber travels with the entry because the entries of one output fiber come
 // from fibers anywhere: searching ptr for each afterwards took 344 us of a
 // 9M-entry transpose, and this kernel takes 60 where it took 56 without.
-template <class PtrT, class P>
+template <class PtrT, class P, int RUN>
 __global__ void __launch_bounds__(FC_THREADS) expand_fibers(int64_t nnz, int64_t nf, const PtrT* __restrict__ ptr,
                                                             const int* __restrict__ idx, int base,
                                                             const char* __restrict__ val, int esz,
                                                             uint32_t* __restrict__ keys, P* __restrict__ payload,
                                                             unsigned long long* __restrict__ hist) {
   __shared__ int s_starts[FC_FIBERS];
-  const int64_t p0 = (int64_t)blockIdx.x * FC_ENTRIES;
-  const int n = nnz - p0 < FC_ENTRIES ? (int)(nnz - p0) : FC_ENTRIES;
+  const int64_t p0 = (int64_t)blockIdx.x * RUN;
+  const int n = nnz - p0 < RUN ? (int)(nnz - p0) : RUN;
   const FiberChunk<PtrT> fibers(ptr, nf, base, p0, n, s_starts);
 #pragma unroll 4
   for (int e = threadIdx.x; e < n; e += FC_THREADS) {
@@ -171,13 +172,22 @@ static int transpose_typed(fgb_ctx* ctx, const fgb_sparse* A, int64_t* out_ptr, 
     const char* val = esz ? (const char*)A->val : nullptr;
     unsigned long long* h = (unsigned long long*)hist;
     const int grid = grid_for(nnz, 256, ctx->num_sms, 8);
-    const unsigned chunks = (unsigned)fc_blocks(nnz);
+    auto expand = [&](auto* payload) {
+      using P = std::remove_pointer_t<decltype(payload)>;
+      auto go = [&](auto run) {
+        constexpr int RUN = decltype(run)::value;
+        expand_fibers<PtrT, P, RUN><<<(unsigned)fc_blocks(nnz, RUN), FC_THREADS, 0, s>>>(nnz, nf, ptr, idx, base, val,
+                                                                                       esz, k_in, payload, h);
+      };
+      if (fc_few(nnz, ctx->num_sms)) go(std::integral_constant<int, FC_FEW>{});
+      else go(std::integral_constant<int, FC_ENTRIES>{});
+    };
     if (wide)
       expand_keys<PtrT><<<grid, 256, 0, s>>>(nnz, idx, base, k_in, (int64_t*)v_in, h);
     else if (psz == 4)
-      expand_fibers<PtrT, uint32_t><<<chunks, FC_THREADS, 0, s>>>(nnz, nf, ptr, idx, base, val, esz, k_in, (uint32_t*)v_in, h);
+      expand((uint32_t*)v_in);
     else
-      expand_fibers<PtrT, uint64_t><<<chunks, FC_THREADS, 0, s>>>(nnz, nf, ptr, idx, base, val, esz, k_in, (uint64_t*)v_in, h);
+      expand((uint64_t*)v_in);
     sort(tmp, tmp_sort, v_in);
     cub::DeviceScan::InclusiveSum(tmp, tmp_scan, hist, out_ptr + 1, ne, s);
     if (wide)

@@ -68,17 +68,18 @@ struct ScaleArgs {
 // local[p] = kept entries of the block's run before entry p, times 2, plus 1
 // where entry p is kept; count[b] = kept entries of run b (count[runs] = 0
 // closes the scan).
-template <class PtrT>
+template <class PtrT, int RUN>
 __global__ void __launch_bounds__(FC_THREADS) scale_flags(ScaleArgs a, const PtrT* __restrict__ ptr,
                                                           int32_t* __restrict__ local,
                                                           int64_t* __restrict__ count) {
-  constexpr int ROUNDS = FC_ENTRIES / FC_THREADS, WARPS = FC_THREADS / 32;
-  static_assert(ROUNDS * WARPS == 64, "two words per lane below");
+  constexpr int ROUNDS = RUN / FC_THREADS, WARPS = FC_THREADS / 32;
+  static_assert(ROUNDS * WARPS <= 64, "two words per lane below");
   __shared__ int s_starts[FC_FIBERS];
-  __shared__ int s_before[ROUNDS * WARPS];
-  const int64_t p0 = (int64_t)blockIdx.x * FC_ENTRIES;
-  const int n = a.nnz - p0 < FC_ENTRIES ? (int)(a.nnz - p0) : FC_ENTRIES;
+  __shared__ int s_before[64];
+  const int64_t p0 = (int64_t)blockIdx.x * RUN;
+  const int n = a.nnz - p0 < RUN ? (int)(a.nnz - p0) : RUN;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (ROUNDS * WARPS < 64 && tid < 64) s_before[tid] = 0;  // the chunk below begins with a barrier
   unsigned kept = 0;  // bit u: entry u * FC_THREADS + tid
   int before[ROUNDS];
   const FiberChunk<PtrT> fibers(ptr, a.nf, a.base, p0, n, s_starts);
@@ -123,15 +124,15 @@ __device__ __forceinline__ T combine(T v, T b, int op) {
   return op == FGB_MAP_DIV ? v / b : v * b;
 }
 
-template <class PtrT>
+template <class PtrT, int RUN>
 __global__ void __launch_bounds__(FC_THREADS) scale_write(ScaleArgs a, const PtrT* __restrict__ ptr,
                                                           const int32_t* __restrict__ local,
                                                           const int64_t* __restrict__ run_pos,
                                                           int32_t* __restrict__ out_idx,
                                                           void* __restrict__ out_val, bool in_f32) {
   __shared__ int s_starts[FC_FIBERS];
-  const int64_t p0 = (int64_t)blockIdx.x * FC_ENTRIES;
-  const int n = a.nnz - p0 < FC_ENTRIES ? (int)(a.nnz - p0) : FC_ENTRIES;
+  const int64_t p0 = (int64_t)blockIdx.x * RUN;
+  const int n = a.nnz - p0 < RUN ? (int)(a.nnz - p0) : RUN;
   const bool by_fiber = (a.by_axis == FGB_AXIS_COL) == (a.csc != 0);
   const FiberChunk<PtrT> fibers(ptr, a.nf, a.base, p0, n, s_starts);
   const int64_t q0 = run_pos[blockIdx.x];
@@ -157,13 +158,13 @@ __global__ void __launch_bounds__(FC_THREADS) scale_write(ScaleArgs a, const Ptr
 }
 
 // out_ptr[f] = the place of fiber f's first entry, for f <= nf.
-template <class PtrT>
+template <class PtrT, int RUN>
 __global__ void scale_ptr(int64_t nnz, int64_t nf, const PtrT* __restrict__ ptr, int base,
                           const int32_t* __restrict__ local, const int64_t* __restrict__ run_pos,
                           int64_t* __restrict__ out_ptr) {
   for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f <= nf; f += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = ld_ptr(ptr, f) - base;
-    out_ptr[f] = p < nnz ? run_pos[p / FC_ENTRIES] + (local[p] >> 1) : run_pos[(nnz + FC_ENTRIES - 1) / FC_ENTRIES];
+    out_ptr[f] = p < nnz ? run_pos[p / RUN] + (local[p] >> 1) : run_pos[(nnz + RUN - 1) / RUN];
   }
 }
 
@@ -171,12 +172,11 @@ static bool value_type_ok(int t) {
   return t == FGB_F64 || t == FGB_F32 || t == FGB_I64 || t == FGB_I32 || t == FGB_BOOL;
 }
 
-template <class PtrT>
-static int sparse_scale_typed(fgb_ctx* ctx, const fgb_sparse* A, const ScaleArgs& a, int64_t* out_ptr,
-                              int32_t* out_idx, void* out_val, int64_t* out_nnz, bool in_f32,
-                              cudaStream_t s) {
+template <class PtrT, int RUN>
+static int sparse_scale_run(fgb_ctx* ctx, const fgb_sparse* A, const ScaleArgs& a, int64_t* out_ptr,
+                            int32_t* out_idx, void* out_val, int64_t* out_nnz, bool in_f32, cudaStream_t s) {
   const PtrT* ptr = (const PtrT*)A->ptr;
-  const int64_t runs = fc_blocks(a.nnz);
+  const int64_t runs = fc_blocks(a.nnz, RUN);
   char* mem = nullptr;  // places within the runs, the runs' counts and their scan
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
@@ -191,11 +191,11 @@ static int sparse_scale_typed(fgb_ctx* ctx, const fgb_sparse* A, const ScaleArgs
   } else {
     int32_t* local = (int32_t*)mem;
     int64_t *count = (int64_t*)(mem + head), *pos = count + (runs + 1);
-    if (runs > 0) scale_flags<PtrT><<<(unsigned)runs, FC_THREADS, 0, s>>>(a, ptr, local, count);
+    if (runs > 0) scale_flags<PtrT, RUN><<<(unsigned)runs, FC_THREADS, 0, s>>>(a, ptr, local, count);
     cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, count, pos, runs + 1, s);
     if (runs > 0)
-      scale_write<PtrT><<<(unsigned)runs, FC_THREADS, 0, s>>>(a, ptr, local, pos, out_idx, out_val, in_f32);
-    scale_ptr<PtrT><<<grid_for(a.nf + 1, 256, ctx->num_sms, 8), 256, 0, s>>>(a.nnz, a.nf, ptr, a.base, local, pos,
+      scale_write<PtrT, RUN><<<(unsigned)runs, FC_THREADS, 0, s>>>(a, ptr, local, pos, out_idx, out_val, in_f32);
+    scale_ptr<PtrT, RUN><<<grid_for(a.nf + 1, 256, ctx->num_sms, 8), 256, 0, s>>>(a.nnz, a.nf, ptr, a.base, local, pos,
                                                                            out_ptr);
     rc = check_launch("fgb_sparse_scale");
     if (rc == FGB_OK) {
@@ -208,6 +208,13 @@ static int sparse_scale_typed(fgb_ctx* ctx, const fgb_sparse* A, const ScaleArgs
   cudaError_t se = cudaStreamSynchronize(s);
   if (rc == FGB_OK && se != cudaSuccess) rc = set_error(FGB_ECUDA, "fgb_sparse_scale: %s", cudaGetErrorString(se));
   return rc;
+}
+
+template <class PtrT>
+static int sparse_scale_typed(fgb_ctx* ctx, const fgb_sparse* A, const ScaleArgs& a, int64_t* out_ptr,
+                              int32_t* out_idx, void* out_val, int64_t* out_nnz, bool in_f32, cudaStream_t s) {
+  auto run = fc_few(a.nnz, ctx->num_sms) ? sparse_scale_run<PtrT, FC_FEW> : sparse_scale_run<PtrT, FC_ENTRIES>;
+  return run(ctx, A, a, out_ptr, out_idx, out_val, out_nnz, in_f32, s);
 }
 
 }  // namespace fgb
