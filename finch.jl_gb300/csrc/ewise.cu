@@ -127,10 +127,12 @@ __device__ __forceinline__ int ew_warp_below(const int* bi, int bbase, int nb, i
 // uniform rows of 16 + 16 69 -> 66.  Not staging where only coordinates are
 // read measured 83 there, 64 warps an SM against 48 66 against 75, and one
 // warp for the longest pairs 322 in place of 155.
-// One thread per fiber stays up to 10 % faster on uniform F64 rows of 5 to 16
-// entries a pair (23.6 us against 25.1 at 5), where its warps never wait for a
-// neighbour, and is 5 to 8 times slower on Zipf rows of the same mean; without
-// the blocks' barriers those took 84 us in place of 71.
+// One thread per fiber and no more stays up to 10 % faster on uniform rows of 2
+// to 8 entries a pair where nothing is written but sums (21.8 us against 24.4
+// at 5, F64): its warps never wait for a neighbour.  It is 5 to 8 times slower
+// on Zipf rows of the same mean; without the block's barrier those took 84 us
+// in place of 71, and a long pair's merge in a function of its own, out of the
+// others' registers, gained nothing.
 // STAGE: false for short fibers, see EW_STAGE_MEAN.
 template <int MODE, bool STAGE, class T, class PA, class PB>
 __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile_k(int64_t nf, int R, Fiber<PA> a, const T* __restrict__ va,
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile
                                                         int32_t* __restrict__ oidx, T* __restrict__ out) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ int s_idx[STAGE ? EW_CAP : 1];
-  __shared__ unsigned s_src[MODE == EW_FILL ? EW_CAP : 1];
+  __shared__ unsigned s_src[MODE == EW_FILL && STAGE ? EW_CAP : 1];
   __shared__ int s_long[EW_THREADS];
   __shared__ int s_nlong;
   __shared__ int s_hits[EW_THREADS / 32];
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile
   const int64_t o0 = MODE == EW_FILL ? optr[f0] : 0;
   const int total = MODE == EW_FILL && staged ? (int)min(optr[f0 + rows] - o0, (int64_t)EW_CAP) : 0;
   for (int k = tid; k < total; k += EW_THREADS) s_src[k] = EW_NONE | EW_NONE << 16;
-  __syncthreads();
+  if (STAGE) __syncthreads();
 
   // Output n of fiber f0 + r (its o-th of `most`), from entries ka / kb of the tile (-1: none).
   auto emit = [&](int64_t at, int64_t most, int64_t o, int c, int64_t ka, int64_t kb) {
@@ -210,15 +212,20 @@ __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile
   };
   if (tid < rows) {
     if (la + lb > EW_LONG) {
-      s_long[atomicAdd(&s_nlong, 1)] = tid;
+      if (STAGE) s_long[atomicAdd(&s_nlong, 1)] = tid;
     } else if constexpr (!STAGE) {
       const int *ai = a.idx + pa, *bi = b.idx + pb;
       const int ea = (int)la, eb = (int)lb, shift = a.base - b.base;
       int i = 0, j = 0, n = 0;
       T acc = T(0);
+      const int64_t at = MODE == EW_FILL ? optr[f0 + tid] : 0;
       while (i < ea && j < eb) {
         const int ca = __ldg(ai + i), cb = __ldg(bi + j) + shift;
         if (ca == cb) {
+          if constexpr (MODE == EW_FILL) {
+            oidx[at + n] = ca - a.base;
+            out[at + n] = wmul(va[pa + i], vb[pb + j]);
+          }
           if constexpr (MODE == EW_REDUCE) acc = fused(va[pa + i], vb[pb + j], acc);
           if constexpr (MODE == EW_SCATTER) atomicAdd(out + (ca - a.base), wmul(va[pa + i], vb[pb + j]));
           ++n;
@@ -234,7 +241,14 @@ __global__ void __launch_bounds__(EW_THREADS, MODE == EW_FILL ? 10 : 16) ew_tile
       merge(a.idx + a0 + pa, a.base, b.idx + b0 + pb, b.base);
     }
   }
-  __syncthreads();
+  if (STAGE) {
+    __syncthreads();
+  } else {  // one barrier where no pair is long
+    const bool is_long = tid < rows && la + lb > EW_LONG;
+    if (!__syncthreads_or(is_long)) return;
+    if (is_long) s_long[atomicAdd(&s_nlong, 1)] = tid;
+    __syncthreads();
+  }
 
   // Lists ai[0, ea) and bi[0, eb) -- entries qa.. and qb.. of the tile -- by a
   // warp, their outputs from `ofs` on: the lane's matches, and its sum.
@@ -415,12 +429,13 @@ __global__ void fold_partials(const T* __restrict__ part, int64_t n, T* __restri
 }
 
 // part[0, n) (with room for EW_FOLD more behind) folded into out[0]: by one
-// block up to 16 partials a thread (one SM reads about 100 GB/s: 2M partials
-// took it 160 us), else in EW_FOLD consecutive shares first.
+// block up to 24 partials a thread (one SM reads about 100 GB/s: 2M partials
+// took it 160 us; 20,000 6 us less than two launches), else in EW_FOLD
+// consecutive shares first.
 constexpr int EW_FOLD = 256;
 template <class T>
 static int fold_all(T* part, int64_t n, T* out, cudaStream_t s) {
-  if (n > 16 * 1024) {
+  if (n > 24 * 1024) {
     fold_partials<T><<<EW_FOLD, 1024, 0, s>>>(part, n, part + n);
     part += n;
     n = EW_FOLD;
@@ -486,13 +501,14 @@ static int ew_rows(const fgb_ctx* ctx, const fgb_sparse* A, const fgb_sparse* B)
   return (int)std::max<int64_t>(r, 1);
 }
 
-// Below this many entries a pair of fibers on average, the modes that write no
-// list read the coordinates where they lie: the copy into shared memory costs
-// a chain of loads and a barrier, and short lists come out of L1.  Row sums of
-// A .* B, F64, 873,496 uniform rows, staged against not: 5 a pair 31.2 / 25.1
-// us, 8 37.0 / 35.2, 12 52.4 / 48.4, 16 63.9 / 65.2, 24 104 / 119; sums
+// Below this many entries a pair of fibers on average, coordinates are read
+// where they lie unless a sum's list is written: the copy into shared memory
+// costs a chain of loads and a barrier, and short lists come out of L1.  Row
+// sums of A .* B, F64, 873,496 uniform rows, staged against not: 5 a pair 31.2
+// / 25.1 us, 8 37.0 / 35.2, 12 52.4 / 48.4, 16 63.9 / 65.2, 24 104 / 119; sums
 // over rows 35.4 / 29.2, 41.6 / 39.5, 59.4 / 56.7, 72.2 / 76.5; Zipf rows
-// 73.8 / 71.4 to 158 / 155 at 16.
+// 73.8 / 71.4 to 158 / 155 at 16; the list of A .* B 96 / 85 at 5, 109 / 99 at
+// 8 (a thread writes the few places that two fibers share itself).
 constexpr double EW_STAGE_MEAN = 14;
 template <int MODE, class T>
 static int ew_tile(fgb_ctx* ctx, const fgb_sparse* A, const fgb_sparse* B, int op, int64_t* cnt, const int64_t* optr,
@@ -501,12 +517,11 @@ static int ew_tile(fgb_ctx* ctx, const fgb_sparse* A, const fgb_sparse* B, int o
   const int R = ew_rows(ctx, A, B);
   const unsigned blocks = (unsigned)((nf + R - 1) / R);
   return with_fibers(A, B, [&](auto fa, auto fb) {
-    if constexpr (MODE != EW_FILL)
-      if ((double)A->nnz + (double)B->nnz < EW_STAGE_MEAN * (double)nf) {
-        ew_tile_k<MODE, false><<<blocks, EW_THREADS, 0, s>>>(nf, R, fa, (const T*)A->val, fb, (const T*)B->val, op,
-                                                             cnt, optr, oidx, out);
-        return check_launch("ew_tile_k");
-      }
+    if ((MODE != EW_FILL || op == FGB_EW_MUL) && (double)A->nnz + (double)B->nnz < EW_STAGE_MEAN * (double)nf) {
+      ew_tile_k<MODE, false><<<blocks, EW_THREADS, 0, s>>>(nf, R, fa, (const T*)A->val, fb, (const T*)B->val, op, cnt,
+                                                           optr, oidx, out);
+      return check_launch("ew_tile_k");
+    }
     ew_tile_k<MODE, true><<<blocks, EW_THREADS, 0, s>>>(nf, R, fa, (const T*)A->val, fb, (const T*)B->val, op, cnt,
                                                         optr, oidx, out);
     return check_launch("ew_tile_k");

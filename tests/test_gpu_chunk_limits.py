@@ -4,9 +4,10 @@ import numpy as np
 import pytest
 import torch
 
+import oracle
 from finchgb import _lib as L
 from finchgb import device as dev
-from helpers import to_dev, to_host, upload
+from helpers import assert_close, to_dev, to_host, upload
 from test_gpu_tiles import csr_of_lengths
 
 pytestmark = pytest.mark.gpu
@@ -38,3 +39,13 @@ def test_runs_of_entries(gpu_lib, over, val):
     assert changed == 0 and np.array_equal(to_host(S.idx), b.idx[kept] - 1)
     assert np.array_equal(to_host(S.val), (v * by[f])[kept])
     assert np.array_equal(np.diff(to_host(S.ptr)), np.bincount(f[kept], minlength=lengths.size))
+
+
+@pytest.mark.parametrize("nf", [1024, 24 * 1024, 24 * 1024 + 1, 40_000])
+def test_fold_of_partials(gpu_lib, nf):
+    """sum(A .* B) over everything: one block's fold, and two levels of it."""
+    rng = np.random.default_rng(nf)
+    b = csr_of_lengths(rng, rng.integers(0, 4, nf), 500, np.float64)
+    want = oracle.ewise_reduce(0, nf, 500, b.ptr, b.idx, b.val, b.ptr, b.idx, b.val)
+    got = to_host(dev.ewise_reduce(0, upload(b), upload(b)))
+    assert_close(got, want, np.abs(want), np.float64)
