@@ -23,6 +23,7 @@
 #include <cub/cub.cuh>
 
 #include "spmm_common.cuh"
+#include "vrow_counts.h"
 
 namespace fgb {
 
@@ -74,17 +75,14 @@ __device__ __forceinline__ bool row_is_light(const RowBands& rb, int P, int T) {
   return true;
 }
 
-// Per row, two counts to a 64-bit word so that two scans place everything
-// (each count's total stays below 2^32): virtual rows and partial-sum slots
-// (rows_slots), fix-up segments (a row's slots in runs of at most VR_SEG) and
-// segment sums (segs_sums; a long row's, one with more than one segment,
-// combined by a second pass).  Totals: virtual rows per band, then long rows.
-// They are summed by block first: an atomic per thread on one address took
-// 200 of the launch's 206 us on the 1M-row matrix.
-__device__ __forceinline__ int64_t vr_pack(int64_t lo, int64_t hi) { return lo | hi << 32; }
-__host__ __device__ __forceinline__ int64_t vr_lo(int64_t w) { return w & 0xffffffffll; }
-__host__ __device__ __forceinline__ int64_t vr_hi(int64_t w) { return (int64_t)((uint64_t)w >> 32); }
-
+// Per row, two counts to a 64-bit word so that two scans place everything:
+// virtual rows and partial-sum slots (rows_slots), fix-up segments (a row's
+// slots in runs of at most VR_SEG) and segment sums (segs_sums; a long row's,
+// one with more than one segment, combined by a second pass).  Totals, in 64
+// bits: virtual rows per band, which say whether the words' halves hold the
+// counts (vrow_fits), then long rows.  They are summed by block first: an
+// atomic per thread on one address took 200 of the launch's 206 us on the
+// 1M-row matrix.
 template <class PtrT>
 __global__ void __launch_bounds__(256) vrow_count_k(int64_t nrows, const PtrT* __restrict__ ptr,
                                                     const int* __restrict__ idx, int base, int T, int P, int64_t W,
@@ -94,8 +92,8 @@ __global__ void __launch_bounds__(256) vrow_count_k(int64_t nrows, const PtrT* _
   __shared__ unsigned long long s_tot[VR_MAX_BANDS + 1];
   if (threadIdx.x <= VR_MAX_BANDS) s_tot[threadIdx.x] = 0;
   __syncthreads();
-  unsigned mine[VR_MAX_BANDS] = {};
-  unsigned nlong = 0;
+  unsigned long long mine[VR_MAX_BANDS] = {};
+  unsigned long long nlong = 0;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nrows;
        r += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b0 = ld_ptr(ptr, r) - base;
@@ -122,7 +120,7 @@ __global__ void __launch_bounds__(256) vrow_count_k(int64_t nrows, const PtrT* _
         const int64_t lb = rb.pos[b + 1] - rb.pos[b];
         const int64_t c = (lb + T - 1) / T;
         nch += c;
-        mine[b] += (unsigned)c;
+        mine[b] += (unsigned long long)c;
       }
       slots = nch - 1;
     }
@@ -131,9 +129,9 @@ __global__ void __launch_bounds__(256) vrow_count_k(int64_t nrows, const PtrT* _
     segs_sums[r] = vr_pack(segs, segs > 1 ? segs : 0);
     nlong += segs > 1;
   }
-  auto add = [&](int t, unsigned v) {
-    v = __reduce_add_sync(0xffffffffu, v);
-    if ((threadIdx.x & 31) == 0 && v) atomicAdd(s_tot + t, (unsigned long long)v);
+  auto add = [&](int t, unsigned long long v) {
+    for (int m = 16; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(s_tot + t, v);
   };
   for (int b = 0; b < P; ++b) add(b, mine[b]);
   add(VR_MAX_BANDS, nlong);
@@ -536,7 +534,7 @@ static int vrow_build_t(fgb_ctx* ctx, const fgb_sparse* A, int T, int P, VrowSch
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail("count");
   const int64_t nv = vr_lo(tot_a), nl = vr_hi(tot_a), nseg = vr_lo(tot_b);
   const int64_t nss = vr_hi(tot_b), nlong = (int64_t)bcnt[VR_MAX_BANDS];
-  if (nv > INT32_MAX || nl > INT32_MAX) {
+  if (!vrow_fits(bcnt, P)) {
     release(false);
     return set_error(FGB_EUNSUPPORTED, "vrow schedule: too many virtual rows");
   }
