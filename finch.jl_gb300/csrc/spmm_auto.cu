@@ -10,10 +10,10 @@
 // the whole block one after another, an equal part per group of the block, the
 // parts added in a fixed order.
 //
-// A row of more entries than two shares hold steps is cut at the shares: the
-// block in whose share it begins writes its part to C, the others leave theirs
-// as carries, and spmm_auto_fixup adds a row's carries in the order of the
-// blocks.  Results are the same run to run.
+// A row of more entries than two shares hold steps is cut at the shares, but in
+// a small product (SA_CUT_BYTES): the block in whose share it begins writes its
+// part to C, the others leave theirs as carries, and spmm_auto_fixup adds a
+// row's carries in the order of the blocks.  Results are the same run to run.
 //
 // A lane keeps 4 sums a column in FP32 (8 for up to 16 columns; FP64, whose
 // pipe waits for the adds, 32 / G, at most 4): at least as many as sub-groups
@@ -45,6 +45,11 @@ constexpr int SA_LIST = 64;  // a share of SA_MAX_STEPS holds the beginnings of 
 // the first wave, at most SA_MAX_STEPS (with 4096, 150,000 rows of 12, k = 64,
 // 79 us in place of 66, 300,000 rows of 4 97 for 80).
 constexpr int64_t SA_MIN_STEPS = 256, SA_MAX_STEPS = 2048;
+// Rows are cut from as many gathered bytes (rows and entries times a row of B):
+// below, the scratch and the second launch cost every call 2.5 us (10,000 rows
+// of 5, k = 64, 11.8 -> 14.6), and a row that had all of the entries keeps one
+// SM for 0.3 ms, in FP64 0.7.
+constexpr double SA_CUT_BYTES = 16.0 * 1024 * 1024;
 // Rows up to this length may be a warp's: 128 entries a group of it, at most
 // 512; none in FP64 where a warp is one group with one sum a lane.
 template <class T, int G>
@@ -287,14 +292,14 @@ __global__ void __launch_bounds__(SA_THREADS) spmm_auto_fixup(int64_t nrows, con
                                                              int64_t ldc) {
   __shared__ T s_sum[SA_THREADS];
   pdl_wait_prev();
-  const int64_t f0 = ld_ptr(ptr, 0);
-  const int64_t per = (ld_ptr(ptr, nrows) - f0 + nrows + nblocks - 1) / nblocks;
   int width = 4;  // columns at a time, a power of two
   while (width < nk && width < SA_THREADS) width *= 2;
   const int runs = SA_THREADS / width, run = threadIdx.x / width;
   for (int64_t w = blockIdx.x; w < nblocks; w += gridDim.x) {  // block-uniform
     const int64_t r = carry_row[w];
     if (r < 0 || (w > 0 && carry_row[w - 1] == r)) continue;
+    const int64_t f0 = ld_ptr(ptr, 0);
+    const int64_t per = (ld_ptr(ptr, nrows) - f0 + nrows + nblocks - 1) / nblocks;
     const int64_t n = (ld_ptr(ptr, r + 1) - f0 - 1 + r) / per - w + 1;  // its carries, up to its last entry's block
     const int64_t len = (n + runs - 1) / runs;
     const int64_t a = w + run * len, b = a + len < w + n ? a + len : w + n;
@@ -330,10 +335,11 @@ static int launch_auto(fgb_ctx* ctx, const fgb_sparse* A, const T* B, int64_t ld
   const int64_t steps = A->nrows + A->nnz;
   const int64_t share = std::clamp(steps / ((int64_t)occ * ctx->num_sms), SA_MIN_STEPS, SA_MAX_STEPS);
   const int grid = (int)std::min<int64_t>((steps + share - 1) / share, INT32_MAX);
-  // no row is cut where the matrix is no wider than that
   const size_t rows_bytes = (sizeof(int64_t) * grid + 255) & ~size_t(255);
   if (need) {
-    *need = grid > 1 && A->ncols > 2 * share ? rows_bytes + sizeof(T) * grid * nk : 0;
+    // no row is as long where the matrix is no wider
+    const bool cut = (double)steps * (double)nk * sizeof(T) >= SA_CUT_BYTES && A->ncols > 2 * share;
+    *need = cut ? rows_bytes + sizeof(T) * grid * nk : 0;
     return FGB_OK;
   }
   int64_t* carry_row = (int64_t*)scratch;
