@@ -98,9 +98,10 @@ struct Semi<SR_PT, double> {
   __device__ static double one() { return 1.0; }
   __device__ static double add(double acc, double t) { return __dadd_rn(acc, t); }
   __device__ static double mul(double a, double x) { return __dmul_rn(x, a); }
-  // Callers pass a compile-time `fm`: with a run-time one the compiler computes
-  // both forms and selects, three FP64 instructions a step where the FP64 pipe
-  // (2 lanes a clock per SM) is what the loops wait for.
+  // The CSR pulls of SpMV and SpMM and SpGEMM's lane tier pass a compile-time
+  // `fm`: with a run-time one (SpGEMM's hash tiers, SDDMM's scalar loop) the
+  // compiler computes both forms and selects, three FP64 instructions a step,
+  // where those pulls wait for the FP64 pipe (2 lanes a clock per SM).
   __device__ static double step(double acc, double a, double x, int fm) {
     if (fm == FM_NOFMA) return __dadd_rn(__dmul_rn(x, a), acc);
     return __fma_rn(x, a, acc);

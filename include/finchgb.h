@@ -249,10 +249,11 @@ FGB_API int fgb_coo_assemble(fgb_ctx* ctx, int64_t nrows, int64_t ncols, int64_t
  * atomic updates of y (order-independent for exact semirings).  With
  * FGB_FINCH_ORDER on a CSR matrix every y[i] is one sequential sum over j
  * ascending, which equals Finch's serial CSC nest bit for bit.  Otherwise a
- * CSR matrix of at least 2^16 rows and stored entries takes the pull that
- * samples its row lengths (lanes per row while no sampled row is long, equal
- * shares of the rows and entries per warp when one is), and a smaller one a
- * fixed number of lanes per row chosen by its mean row length. */
+ * CSR matrix whose rows and stored entries sum to 2^16 or more takes the pull
+ * that samples its row lengths (lanes per row while no sampled row is long,
+ * equal shares of the rows and entries per warp when one is, or when rows are
+ * long on average), and a smaller one a fixed number of lanes per row chosen by
+ * its mean row length.  Float results are the same run to run. */
 FGB_API int fgb_spmv(fgb_ctx* ctx, int semiring, const fgb_sparse* A, const void* x, int x_t, void* y,
              int y_t, unsigned flags, void* stream);
 
