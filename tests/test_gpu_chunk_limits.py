@@ -49,3 +49,14 @@ def test_fold_of_partials(gpu_lib, nf):
     want = oracle.ewise_reduce(0, nf, 500, b.ptr, b.idx, b.val, b.ptr, b.idx, b.val)
     got = to_host(dev.ewise_reduce(0, upload(b), upload(b)))
     assert_close(got, want, np.abs(want), np.float64)
+
+
+@pytest.mark.parametrize("m", [63, 64, 65, 128])
+def test_spgemm_blocks_of_rows(gpu_lib, m):
+    """Rows merged by one thread each, 64 a block: a block that is full, one row
+    short and one row over, the last row another tier's."""
+    rng = np.random.default_rng(m)
+    A, B = csr_of_lengths(rng, [5] * (m - 1) + [40], 300, np.float64), csr_of_lengths(rng, np.full(300, 7), 900, np.float64)
+    ptr, idx, val = dev.spgemm(upload(A), upload(B)).to_host()
+    wp, wi, wv = oracle.spgemm_csr(m, 900, A.ptr, A.idx, A.val, B.ptr, B.idx, B.val, fma=True)
+    assert np.array_equal(ptr, wp) and np.array_equal(idx, wi) and np.array_equal(val, wv)
