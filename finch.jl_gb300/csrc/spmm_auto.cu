@@ -46,10 +46,11 @@ constexpr int SA_LIST = 64;  // a share of SA_MAX_STEPS holds the beginnings of 
 // 79 us in place of 66, 300,000 rows of 4 97 for 80).
 constexpr int64_t SA_MIN_STEPS = 256, SA_MAX_STEPS = 2048;
 // Rows are cut from as many gathered bytes (rows and entries times a row of B):
-// below, the scratch and the second launch cost every call 2.5 us (10,000 rows
-// of 5, k = 64, 11.8 -> 14.6), and a row that had all of the entries keeps one
-// SM for 0.3 ms, in FP64 0.7.
-constexpr double SA_CUT_BYTES = 16.0 * 1024 * 1024;
+// below, the scratch and the second launch cost a call whose host side takes
+// as long as its kernel 3 us (10,000 rows of 5, k = 64, 11.8 -> 14.6; through
+// lazy tensors 22,828 rows of 5, k = 32, FP64, 34 -> 38), and a row that had
+// all of the entries keeps one SM for 1.1 ms at most, in FP64 2.6.
+constexpr double SA_CUT_BYTES = 64.0 * 1024 * 1024;
 // Rows up to this length may be a warp's: 128 entries a group of it, at most
 // 512; none in FP64 where a warp is one group with one sum a lane.
 template <class T, int G>

@@ -109,9 +109,10 @@ def test_spmm_hub_rows_are_cut(gpu_lib, nk, dtype):
     entries at most (2,048) share a sum with the first, and the parts of every
     row meet in a fixed order; rows before, between and after them, a second
     slab of columns, accumulating into strided rows."""
+    hub = {32: 200_000, 64: 120_000}.get(nk, 60_000)  # from nk = 32 on 64 MB of gathers, the size from which rows are cut
     lengths = np.full(3000, 5)
-    lengths[[0, 700, 701, 2999]] = (60_000, 30_000, 21_000, 60_000)
-    n = 70_000
+    lengths[[0, 700, 701, 2999]] = (hub, hub // 2, hub // 3 + 1000, hub)
+    n = hub + 10_000
     b, _ = swallowing(lengths, n, dtype)
     big = 2.0 ** (24 if dtype == np.float32 else 53)
     B = torch.ones((n, nk + 4), dtype=torch.float32 if dtype == np.float32 else torch.float64, device="cuda")[:, :nk]
